@@ -70,7 +70,7 @@ def draw(rng):
     if op == "rollup":  # from a few shard hashes to a shard of some thousand records
         return {"op": op, "leaves": _log_uniform(rng, 10, 4000)}
     if op in ("sha256", "sha512"):  # record bytes, up to a large record set
-        return {"op": op, "bytes": rng.choice([0, _log_uniform(rng, 16, 4000), rng.randrange(1, 600), rng.randrange(40, 4000)])}
+        return {"op": op, "bytes": rng.choice([_log_uniform(rng, 16, 4000), rng.randrange(1, 600), rng.randrange(40, 4000)])}
     if op == "rsa":
         return {"op": op, "records": _log_uniform(rng, 2, 32)}
     if op == "ecdsa":  # chains shorter than the full scalar are the AIR's own small sizes
@@ -91,9 +91,9 @@ def draw(rng):
         cols = rng.choice([1, 2, 6, 12, 18, 48, 64, _log_uniform(rng, 1, 128)])
         return {"op": op, "cols": cols, "leaves": _log_uniform(rng, 64, (1 << 26) // cols)}
     if op == "stir":
-        return {"op": op, "log_n": rng.randrange(9, 22)}
+        return {"op": op, "log_n": rng.choice([*range(9, 20), 21])}
     blowup = rng.choice([4, 32])  # at least 4096 points: below, the default gate leaves the constraints out
-    return {"op": op, "log_n": rng.randrange(12 - (blowup.bit_length() - 1), 13), "blowup": blowup}
+    return {"op": op, "log_n": rng.randrange(12 - (blowup.bit_length() - 1), 12 if blowup == 32 else 15), "blowup": blowup}
 
 
 # ------------------------------------------------------------------ inputs
