@@ -10,6 +10,7 @@
 #include "ed25519_prover.hpp"
 #include "merge.cuh"
 #include "merkle.cuh"
+#include "ntt_tc.cuh"
 #include "p256.hpp"
 #include "p256_prover.hpp"
 #include "prover.hpp"
@@ -36,6 +37,7 @@ int guarded(sg_ctx* c, F&& f) {
   try {
     if (cudaSetDevice(c->device) != cudaSuccess) return fail(c, SG_ECUDA, "cudaSetDevice failed");
     f();
+    if (sg::ntt_tc_timed_out()) return fail(c, SG_ECUDA, "a bounded wait in a transform kernel ran out");
     c->err.clear();
     return SG_OK;
   } catch (const sg::SgError& e) {

@@ -31,6 +31,7 @@
 #include "gl.cuh"
 #include "keccak.cuh"
 #include "ntt.cuh"
+#include "ntt_tc.cuh"
 
 namespace sg {
 namespace {
@@ -578,6 +579,20 @@ const uint64_t* coset_twist_table(const NttTables& t, int log_n, cudaStream_t s)
 // per-size table (shared through L2) instead of building per-CTA factors
 constexpr uint32_t kPassTabMinCols = 8;
 
+// log2 of the expansion E of a zero-padded transform: only the first N / E inputs can be non-zero
+int log_expansion(uint64_t n_valid, int log_n) {
+  int e = 0;
+  while (e < log_n && n_valid <= (1ull << (log_n - e - 1))) ++e;
+  return e;
+}
+
+// outputs j = q jq + x jx + S i1 at stride out_j
+void tc_out(TcPass* a, uint64_t out_j) {
+  a->out_q = a->jq * out_j;
+  a->out_x = a->jx * out_j;
+  a->out_i = out_j << a->log_s;
+}
+
 int sparse_nz_for(uint64_t n_valid, uint64_t N, uint64_t n_lo, uint64_t M) {
   if (n_valid >= N || M < 16) return 0;  // dense, or a pass without a radix-16 first stage
   const uint64_t m_nz = (n_valid + n_lo - 1) / n_lo, G = M / 16;
@@ -651,16 +666,18 @@ cudaError_t ntt_tables_init(NttTables* t) {
   *t = ntt_tables_view(dev);
   t->owned = true;
   t->pass_tables = true;
+  t->tc = tc_cache_new();
   return cudaSuccess;
 }
 
 void ntt_tables_free(NttTables* t) {
   if (t->owned && t->d_fwd_st) cudaFree(t->d_fwd_st);
+  if (t->owned) tc_cache_free(t->tc);
   *t = NttTables{};
 }
 
 bool ntt_coset_eval_ok(int log_m, int log_b) {
-  return log_m >= 1 && log_m <= 12 && log_b >= pass_log_k(log_m) && log_m + log_b <= kMaxLogN;
+  return log_m >= 1 && log_m <= 12 && (ntt_tc_ok(log_m) || log_b >= pass_log_k(log_m)) && log_m + log_b <= kMaxLogN;
 }
 
 // Coset t < B of the evaluation domain is the DFT_M of c_m * g^m * w_N^{t m}:
@@ -673,6 +690,21 @@ cudaError_t ntt_coset_eval(const NttTables& t, const uint64_t* coef, uint64_t* o
   if (!ntt_coset_eval_ok(log_m, log_b)) return cudaErrorInvalidValue;
   if (n_cols == 0) return cudaSuccess;
   const uint64_t M = 1ull << log_m, B = 1ull << log_b;
+  if (ntt_tc_ok(log_m)) {
+    TcPass p = ntt_tc_args(log_m, log_b);
+    p.in = coef;
+    p.out = out;
+    p.in_lane = M;
+    p.in_m = 1;
+    p.out_lane = M * B;
+    tc_out(&p, 1);
+    p.n_lanes = n_cols;
+    p.in_valid = M;
+    p.pre = pre ? *pre : PowSpec{};
+    if (ntt_tc_tables(t, &p, false, s)) return ntt_tc_pass(p, false, s);
+  }
+  // fewer cosets than a lane-per-coset pass's lanes
+  if (log_b < pass_log_k(log_m)) return t.tc ? cudaErrorMemoryAllocation : cudaErrorInvalidValue;
   PassArgs a = base_args(t, false);
   a.pre = pre ? *pre : PowSpec{};
   a.in = coef;
@@ -719,6 +751,18 @@ int ntt_split(int log_n, bool padded) {
   return tuned ? tuned : log_n / 2;
 }
 
+// The split of one transform: the pinned one, else the one whose passes both run on
+// the tensor cores (2^8 .. 2^10 points each, 2^v = N / 2^le inputs), else one with the
+// larger pass on them, else log N / 2.
+static int ntt_split(int log_n, bool padded, int le, bool tc) {
+  const int tuned = g_split[log_n][padded ? 1 : 0].load(), v = log_n - le;
+  if (tuned) return tuned;
+  if (tc && v >= 16 && v <= 20) return v / 2;
+  if (tc && v >= 11 && v < 16) return v - 8;
+  if (tc && le == 0 && log_n <= 22) return 10;
+  return log_n / 2;
+}
+
 void ntt_set_split(int log_n, bool padded, int log_n1) {
   if (log_n >= 13 && log_n <= 24) g_split[log_n][padded ? 1 : 0].store(log_n1);
 }
@@ -738,6 +782,20 @@ cudaError_t ntt_batch(const NttTables& t, const uint64_t* in, uint64_t* out, uin
   }
   const uint64_t ninv = inverse ? gl::inv(N) : 1;
   const PowSpec none{};
+  if (ntt_tc_ok(log_n)) {
+    TcPass p = ntt_tc_args(log_n, 0);
+    p.in = in;
+    p.out = out;
+    p.in_lane = in_stride;
+    p.in_m = 1;
+    p.out_lane = out_stride;
+    tc_out(&p, 1);
+    p.n_lanes = n_cols;
+    p.in_valid = n_valid;
+    p.pre = pre ? *pre : none;
+    p.scale = ninv;
+    if (ntt_tc_tables(t, &p, inverse, s)) return ntt_tc_pass(p, false, s);
+  }
   if (log_n <= 12) {
     // one pass; the lanes are the columns (a length-1 "transform" is the identity
     // pass, used only to apply pre)
@@ -757,7 +815,21 @@ cudaError_t ntt_batch(const NttTables& t, const uint64_t* in, uint64_t* out, uin
   }
   if (!scratch) return cudaErrorInvalidValue;
   if (log_n <= 24) {
-    const int l1 = ntt_split(log_n, n_valid < N), l2 = log_n - l1;
+    const int le = log_expansion(n_valid, log_n);  // zero padding: pass 1 evaluates 2^le outputs per input
+    int l1 = ntt_split(log_n, n_valid < N, le, t.tc != nullptr), l2 = log_n - l1;
+    TcPass p1 = ntt_tc_args(l2 - le, le), p2 = ntt_tc_args(l1, 0);
+    if (pre) p1.pre = *pre;
+    p1.flat_m = 1ull << l1;
+    p2.scale = ninv;
+    bool tc1 = ntt_tc_ok(l2 - le), tc2 = ntt_tc_ok(l1);
+    if (tc1) tc1 = ntt_tc_tables(t, &p1, inverse, s);
+    if (tc2) tc2 = ntt_tc_tables(t, &p2, inverse, s);
+    if (!tc1 && l2 > 12) {  // no room for the tables: the split whose passes need none
+      if (tc2) ntt_tc_drop(p2, s);
+      tc2 = false;
+      l1 = log_n / 2;
+      l2 = log_n - l1;
+    }
     const uint64_t N1 = 1ull << l1, N2 = 1ull << l2;
     // pass 1: DFT_{N2} over k2 (stride N1), lanes k1; transposed store into scratch
     PassArgs a = base_args(t, inverse);
@@ -778,13 +850,51 @@ cudaError_t ntt_batch(const NttTables& t, const uint64_t* in, uint64_t* out, uin
     // enough columns share the table: then the CTAs of one lane group run over all
     // columns back to back and read its entries from L2 (one load and one product
     // per element instead of two shared loads and two products).
-    if (t.pass_tables && (!pass_tw_in_smem(l2) || n_cols >= kPassTabMinCols)) {
+    if (!tc1 && t.pass_tables && (!pass_tw_in_smem(l2) || n_cols >= kPassTabMinCols)) {
       a.tw_tab = pass_twiddle_table(t, log_n, l1, inverse, s);
       a.cols_fast = a.tw_tab && pass_tw_in_smem(l2) && (N1 >> pass_log_k(l2)) <= 65535;
     }
     a.pre = pre ? *pre : none;
-    cudaError_t e = launch_pass_dyn(l2, a, inverse, n_cols, s);
-    if (e != cudaSuccess) return e;
+    cudaError_t e;
+    if (tc1) {
+      p1.in = in;
+      p1.out = scratch;
+      p1.in_col = in_stride;
+      p1.out_col = N;
+      p1.in_lane = 1;
+      p1.in_m = N1;
+      p1.out_lane = 1;
+      tc_out(&p1, N1);
+      p1.n_lanes = (uint32_t)N1;
+      p1.n_y = n_cols;
+      p1.flat_lane = 1;
+      p1.in_valid = n_valid;
+      p1.pt_log = log_n;
+      p1.canon = !tc2;
+      p1.strided = true;
+      e = ntt_tc_pass(p1, true, s);
+    } else {
+      e = launch_pass_dyn(l2, a, inverse, n_cols, s);
+    }
+    if (e != cudaSuccess) {
+      if (tc2) ntt_tc_drop(p2, s);
+      return e;
+    }
+    if (tc2) {
+      p2.in = scratch;
+      p2.out = out;
+      p2.in_col = N;
+      p2.out_col = out_stride;
+      p2.in_lane = N1;
+      p2.in_m = 1;
+      p2.out_lane = 1;
+      tc_out(&p2, N2);
+      p2.n_lanes = (uint32_t)N2;
+      p2.n_y = n_cols;
+      p2.in_valid = N;
+      p2.strided = true;
+      return ntt_tc_pass(p2, true, s);
+    }
     // pass 2: DFT_{N1} over contiguous rows, lanes i2; natural-order store
     PassArgs b = base_args(t, inverse);
     b.in = scratch;

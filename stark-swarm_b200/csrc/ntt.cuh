@@ -15,6 +15,7 @@ static constexpr int kTwBaseLog = 28;   // global twiddles are powers of w28 = w
 static constexpr int kTwSplit = 14;     // w28^E = lo[E & (2^14-1)] * hi[E >> 14]
 static constexpr int kTwEntries = 1 << kTwSplit;
 
+struct TcCache;
 struct NttTables {
   // Per direction (forward: w, inverse: w^-1):
   //   st[i] = w_4096^i (i < 4096)       — in-CTA Stockham stage twiddles
@@ -30,6 +31,9 @@ struct NttTables {
   // table kept for the process (pass_twiddle_table); off for tables made by
   // ntt_tables_view (callers that must not allocate).
   bool pass_tables = false;
+  // byte matrices of the tensor-core passes (ntt_tc.cu), built per shape on first use;
+  // null for callers that must not allocate
+  TcCache* tc = nullptr;
 };
 
 // Elements of one direction's block: st (4096) + lo + hi.

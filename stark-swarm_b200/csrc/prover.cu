@@ -13,6 +13,7 @@
 #include "gl.cuh"
 #include "merge.cuh"
 #include "merkle.cuh"
+#include "ntt_tc.cuh"
 #include "rsa_air.cuh"
 #include "prover.hpp"
 #include "hash_air.hpp"
@@ -86,7 +87,7 @@ struct ShiftTables {
 // scratch buffer the size of the LDE.
 bool lde_by_cosets(uint64_t n_trace, uint64_t blowup) {
   const int lm = (int)log2_exact(n_trace), lb = (int)log2_exact(blowup);
-  return lm + lb > 12 && ntt_coset_eval_ok(lm, lb);
+  return (lm + lb > 12 || ntt_tc_ok(lm)) && ntt_coset_eval_ok(lm, lb);
 }
 
 // iNTT of w columns into coef, then the zero-padded forward transform into d_out,
@@ -1058,17 +1059,34 @@ struct StirStreamScope {
 
 }  // namespace
 
+// A proof whose transforms ran out of a bounded wait is not handed out.
+static void check_waits() {
+  if (ntt_tc_timed_out()) throw SgError{SG_ECUDA, "a bounded wait in a transform kernel ran out"};
+}
+
 std::vector<uint8_t> stir_prove_device(sg_ctx* c, const uint64_t* d_f0, uint64_t n0, const sg_fri_params& p) {
-  if (!c->stir_stream) return stir_prove_on_stream(c, d_f0, n0, p);
-  StirStreamScope scope(c);
-  return stir_prove_on_stream(c, d_f0, n0, p);
+  std::vector<uint8_t> proof;
+  if (!c->stir_stream) {
+    proof = stir_prove_on_stream(c, d_f0, n0, p);
+  } else {
+    StirStreamScope scope(c);
+    proof = stir_prove_on_stream(c, d_f0, n0, p);
+  }
+  check_waits();
+  return proof;
 }
 
 std::vector<std::vector<uint8_t>> stir_prove_group(sg_ctx* c, const uint64_t* d_f0, uint64_t g_f0, uint64_t n0,
                                                    const std::vector<sg_fri_params>& ps) {
-  if (!c->stir_stream) return stir_prove_group_on_stream(c, d_f0, g_f0, n0, ps);
-  StirStreamScope scope(c);
-  return stir_prove_group_on_stream(c, d_f0, g_f0, n0, ps);
+  std::vector<std::vector<uint8_t>> proofs;
+  if (!c->stir_stream) {
+    proofs = stir_prove_group_on_stream(c, d_f0, g_f0, n0, ps);
+  } else {
+    StirStreamScope scope(c);
+    proofs = stir_prove_group_on_stream(c, d_f0, g_f0, n0, ps);
+  }
+  check_waits();
+  return proofs;
 }
 
 // ------------------------------------------------------------------ HashRollup pipeline

@@ -1,0 +1,64 @@
+"""The tensor-core NTT passes (ntt_tc.cu) against the oracle, bit-exact, at the sizes
+where their tiling can go wrong: one lane, a tile's lanes and one more, more tiles than a
+CTA keeps in flight, more than one chunk, both passes of a four-step transform, zero
+padding, and element values whose bytes make the digit sums extreme."""
+import numpy as np
+import pytest
+
+import oracle_lib as O
+
+pytestmark = pytest.mark.gpu
+P = O.P
+
+
+def field(rng, cols, n, kind="random"):
+    if kind == "random":
+        return rng.integers(0, P, size=(cols, n), dtype=np.uint64)
+    # values of all-ones bytes (high word), the largest element, zero and one
+    return rng.choice(np.array([0, 1, P - 1, 0xFFFFFFFEFFFFFFFF, 0xFFFFFFFF], dtype=np.uint64), size=(cols, n))
+
+
+# one pass: 2^8 and 2^9 have 8 lanes a tile, 2^10 has 4
+@pytest.mark.parametrize("log_n", [8, 9, 10])
+@pytest.mark.parametrize("cols", [1, 4, 5, 8, 9, 37])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_one_pass(ctx, log_n, cols, inverse):
+    rng = np.random.default_rng(cols * 100 + log_n)
+    for kind in ("random", "extreme"):
+        x = field(rng, cols, 1 << log_n, kind)
+        got = ctx.ntt(x, log_n, inverse)
+        for c in (0, cols // 2, cols - 1):
+            assert np.array_equal(got[c], O.ntt(x[c], inverse)), (kind, c)
+
+
+# two passes: both on the tensor cores (2^16 .. 2^20), or the first one only
+@pytest.mark.parametrize("log_n,cols", [(13, 3), (14, 1), (15, 2), (16, 1), (16, 5), (17, 2), (18, 1), (19, 3), (20, 1),
+                                        (21, 1), (22, 1)])
+def test_two_passes(ctx, log_n, cols):
+    rng = np.random.default_rng(log_n)
+    x = field(rng, cols, 1 << log_n, "extreme" if log_n % 2 else "random")
+    for inverse in (False, True):
+        got = ctx.ntt(x, log_n, inverse)
+        for c in range(cols):
+            assert np.array_equal(got[c], O.ntt(x[c], inverse)), (inverse, c)
+
+
+# LDE: coset evaluation in one pass (traces of 2^8 .. 2^10 rows), and padded two-pass
+# transforms (2^11 .. 2^16 rows), with and without a coset shift
+@pytest.mark.parametrize("w,log_n,blowup,shift", [
+    (1, 8, 2, 1), (9, 8, 4, 7), (17, 8, 32, 1), (8, 9, 2, 3), (3, 9, 16, 1), (5, 10, 2, 7), (1, 10, 4, 1), (33, 10, 32, 5),
+    (2, 11, 4, 7), (3, 12, 32, 1), (1, 13, 2, 1), (2, 14, 8, 7), (1, 15, 16, 1), (2, 16, 4, 7), (1, 17, 8, 1), (1, 8, 1024, 7),
+])
+def test_lde(ctx, w, log_n, blowup, shift):
+    rng = np.random.default_rng(w + 10 * log_n)
+    tr = field(rng, w, 1 << log_n)
+    assert np.array_equal(ctx.lde(tr, blowup, shift), O.lde(tr, blowup, shift))
+
+
+def test_repeated_calls_and_tables(ctx):
+    """A shape's tables are built once and shared by later calls, another shift in between."""
+    rng = np.random.default_rng(5)
+    tr = field(rng, 12, 256)
+    want = {s: O.lde(tr, 8, s) for s in (1, 7, 11)}
+    for s in (1, 7, 1, 11, 1, 7):
+        assert np.array_equal(ctx.lde(tr, 8, s), want[s]), s
