@@ -593,6 +593,54 @@ void tc_out(TcPass* a, uint64_t out_j) {
   a->out_i = out_j << a->log_s;
 }
 
+// Between two tensor-core passes the data lies in blocks of b = the writing pass's tile
+// lanes k: [k / b][j][k % b]. The writer then stores 8 b bytes times the adjacent j of a
+// warp, 256 bytes on end, and the reader reads at least 128 on end, where [j][k] would have
+// both move 32-byte pieces (64 x 2^20 x 8: 9.0 -> 8.0 ms with the scratch in blocks and the
+// first pass's twiddles from its lane tables, then 7.0 with the coefficients in blocks too).
+//
+// First pass of a four-step transform N = 2^l1 N2: lanes k1 < 2^l1, outputs j < N2 at
+// out[j 2^l1 + k1], or in blocks of `block` lanes.
+void tc_first(TcPass* p, const uint64_t* in, uint64_t in_col, uint64_t* out, int log_n, int l1, uint32_t n_cols,
+              int block) {
+  const uint64_t N1 = 1ull << l1, N2 = 1ull << (log_n - l1);
+  p->in = in;
+  p->out = out;
+  p->in_col = in_col;
+  p->out_col = 1ull << log_n;
+  p->in_lane = 1;
+  p->in_m = N1;
+  p->out_lane = 1;
+  tc_out(p, block ? block : N1);
+  p->out_g = N2 * block;
+  p->n_lanes = (uint32_t)N1;
+  p->n_y = n_cols;
+  p->flat_lane = 1;
+  p->in_valid = 1ull << log_n;
+  p->pt_log = log_n;
+  p->canon = !block;
+  p->strided = true;
+}
+// Second pass: lanes j < N2 of 2^l1 points, inputs as tc_first left them, natural-order outputs.
+void tc_second(TcPass* p, const uint64_t* in, uint64_t* out, uint64_t out_col, int log_n, int l1, uint32_t n_cols,
+               int block) {
+  const uint64_t N1 = 1ull << l1, N2 = 1ull << (log_n - l1);
+  p->in = in;
+  p->out = out;
+  p->in_col = 1ull << log_n;
+  p->out_col = out_col;
+  p->in_lane = block ? block : N1;
+  p->in_m = 1;
+  p->in_block = block;
+  p->in_h = N2 * block;
+  p->out_lane = 1;
+  tc_out(p, N2);
+  p->n_lanes = (uint32_t)N2;
+  p->n_y = n_cols;
+  p->in_valid = N1;
+  p->strided = true;
+}
+
 int sparse_nz_for(uint64_t n_valid, uint64_t N, uint64_t n_lo, uint64_t M) {
   if (n_valid >= N || M < 16) return 0;  // dense, or a pass without a radix-16 first stage
   const uint64_t m_nz = (n_valid + n_lo - 1) / n_lo, G = M / 16;
@@ -857,21 +905,8 @@ cudaError_t ntt_batch(const NttTables& t, const uint64_t* in, uint64_t* out, uin
     a.pre = pre ? *pre : none;
     cudaError_t e;
     if (tc1) {
-      p1.in = in;
-      p1.out = scratch;
-      p1.in_col = in_stride;
-      p1.out_col = N;
-      p1.in_lane = 1;
-      p1.in_m = N1;
-      p1.out_lane = 1;
-      tc_out(&p1, N1);
-      p1.n_lanes = (uint32_t)N1;
-      p1.n_y = n_cols;
-      p1.flat_lane = 1;
+      tc_first(&p1, in, in_stride, scratch, log_n, l1, n_cols, tc2 ? ntt_tc_lanes(l2 - le) : 0);
       p1.in_valid = n_valid;
-      p1.pt_log = log_n;
-      p1.canon = !tc2;
-      p1.strided = true;
       e = ntt_tc_pass(p1, true, s);
     } else {
       e = launch_pass_dyn(l2, a, inverse, n_cols, s);
@@ -881,18 +916,7 @@ cudaError_t ntt_batch(const NttTables& t, const uint64_t* in, uint64_t* out, uin
       return e;
     }
     if (tc2) {
-      p2.in = scratch;
-      p2.out = out;
-      p2.in_col = N;
-      p2.out_col = out_stride;
-      p2.in_lane = N1;
-      p2.in_m = 1;
-      p2.out_lane = 1;
-      tc_out(&p2, N2);
-      p2.n_lanes = (uint32_t)N2;
-      p2.n_y = n_cols;
-      p2.in_valid = N;
-      p2.strided = true;
+      tc_second(&p2, scratch, out, out_stride, log_n, l1, n_cols, tc1 ? ntt_tc_lanes(l2 - le) : 0);
       return ntt_tc_pass(p2, true, s);
     }
     // pass 2: DFT_{N1} over contiguous rows, lanes i2; natural-order store
@@ -969,6 +993,46 @@ cudaError_t ntt_batch(const NttTables& t, const uint64_t* in, uint64_t* out, uin
   c.in_valid = N;
   c.scale = ninv;
   return launch_pass_dyn(la, c, inverse, n_cols, s);
+}
+
+// Inverse transform and zero-padded forward transform with the coefficients between them
+// in blocks (tc_first's and tc_second's): both ends of that buffer then move whole pieces.
+cudaError_t ntt_lde(const NttTables& t, const uint64_t* in, uint64_t* coef, uint64_t* out, uint32_t n_cols, int log_n,
+                    int log_b, uint64_t* scratch, cudaStream_t s, const PowSpec* pre) {
+  const int log_e = log_n + log_b, l1 = log_n / 2, l2 = log_n - l1;
+  if (!t.tc || !ntt_tc_ok(l1) || !ntt_tc_ok(l2) || log_b < 1 || log_e > 24 || !scratch || n_cols == 0 ||
+      g_split[log_n][0].load() || g_split[log_e][1].load())
+    return cudaErrorNotSupported;
+  const uint64_t n = 1ull << log_n;
+  TcPass p[4] = {ntt_tc_args(l2, 0), ntt_tc_args(l1, 0), ntt_tc_args(l1, log_b), ntt_tc_args(l2, 0)};
+  p[0].flat_m = 1ull << l1;
+  p[1].scale = gl::inv(n);
+  p[2].flat_m = 1ull << l2;
+  if (pre) p[2].pre = *pre;
+  for (int k = 0; k < 4; ++k)
+    if (!ntt_tc_tables(t, &p[k], k < 2, s)) {
+      for (int i = 0; i < k; ++i) ntt_tc_drop(p[i], s);
+      return cudaErrorNotSupported;
+    }
+  // the second and the third pass have the same points per lane, so the same lanes a tile
+  const int block = ntt_tc_lanes(l1);
+  tc_first(&p[0], in, n, scratch, log_n, l1, n_cols, ntt_tc_lanes(l2));
+  tc_second(&p[1], scratch, coef, n, log_n, l1, n_cols, ntt_tc_lanes(l2));
+  p[1].out_g = block << l1;
+  tc_out(&p[1], block);
+  tc_first(&p[2], coef, n, scratch, log_e, l2, n_cols, block);
+  p[2].in_g = block << l1;
+  p[2].in_m = block;
+  p[2].in_valid = n;
+  tc_second(&p[3], scratch, out, 1ull << log_e, log_e, l2, n_cols, block);
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < 4; ++k) {
+    if (e == cudaSuccess)
+      e = ntt_tc_pass(p[k], true, s);
+    else
+      ntt_tc_drop(p[k], s);
+  }
+  return e;
 }
 
 // ------------------------------------------------------------------ fused LDE -> leaf hash

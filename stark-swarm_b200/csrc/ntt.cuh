@@ -86,6 +86,14 @@ cudaError_t ntt_batch(const NttTables& t, const uint64_t* in, uint64_t* out, uin
                       uint64_t out_stride, int log_n, bool inverse, uint64_t n_valid, uint64_t* scratch,
                       cudaStream_t s, const PowSpec* pre = nullptr);
 
+// The LDE of n_cols columns of 2^log_n values (column stride 2^log_n) onto 2^(log_n + log_b)
+// points, as ntt_batch's inverse and then its zero-padded forward transform with `pre`, for
+// traces of 2^16 .. 2^20 rows; coef (n_cols 2^log_n elements) holds the coefficients in an
+// order of its own. cudaErrorNotSupported (nothing done) when these transforms do not run
+// on the tensor cores or a split is pinned. scratch: ntt_scratch_elems(n_cols, log_n + log_b).
+cudaError_t ntt_lde(const NttTables& t, const uint64_t* in, uint64_t* coef, uint64_t* out, uint32_t n_cols, int log_n,
+                    int log_b, uint64_t* scratch, cudaStream_t s, const PowSpec* pre = nullptr);
+
 // Evaluate n_cols polynomials of degree < M = 2^log_m (coefficients contiguous,
 // column stride M) on the N = M * 2^log_b points g * w_N^j in natural order
 // (column stride N) in one pass, without scratch: a forward transform of the

@@ -19,7 +19,7 @@
 // active 25 % (R1 = 16) to 45 % (R1 = 32) of the time, HBM 20-30 %. Measured (one call, device
 // tensors, before = the radix-16 butterfly passes of ntt.cu, after): LDE of 4099 x 1024
 // points x 32: 1666 -> 600 us; 20000 x 256 x 32: 1588 -> 595 us; 64 x 2^20 x 8:
-// 14.7 -> 9.1 ms; inverse 6 x 2^20: 178 -> 128 us; one column of 2^8: 25 -> 19 us.
+// 14.7 -> 7.0 ms; inverse 6 x 2^20: 178 -> 130 us; one column of 2^8: 25 -> 19 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -187,7 +187,9 @@ __device__ __forceinline__ void issue(uint32_t d, uint32_t a, uint32_t b, uint32
   __syncwarp();
 }
 
-template <int LR1, int LR2>
+// PT (pass twiddle of a four-step transform's first pass): 0 none, canonical results; 1 formed
+// as a geometric sequence; 2 from tables of the tile's lanes, shared by many columns
+template <int LR1, int LR2, int PT>
 struct Shape {
   static constexpr int R1 = 1 << LR1, R2 = 1 << LR2;
   static constexpr int L = kRows / R1;                                     // lanes of a tile
@@ -201,7 +203,10 @@ struct Shape {
   static constexpr uint32_t B1_BYTES = 8 * R1 * 8 * R2, B2_BYTES = 8 * R1 * 8 * R1;
   static constexpr uint32_t T_BYTES = R1 * R1 * 8;
   static constexpr uint32_t Q_BYTES = B1_BYTES + T_BYTES;                  // a chunk's tables
-  static constexpr uint32_t SMEM = B2_BYTES + Q_BYTES + GROUPS * A_BYTES + 64 + 1024;
+  // twiddles in shared memory: the chunk's [x][m1], or for PT = 2 [x][row] times w_N^(j' lane)
+  // and the factors w_N^(S i1 lane) at [i1][l]
+  static constexpr uint32_t TW_BYTES = PT == 2 ? kRows * R1 * 8 + L * R1 * 8 : T_BYTES;
+  static constexpr uint32_t SMEM = B2_BYTES + B1_BYTES + TW_BYTES + GROUPS * A_BYTES + 64 + 1024;
 };
 
 // byte matrix entries of one (output, input) pair: out[d] byte b = byte d of v 2^(8b) mod p
@@ -271,11 +276,9 @@ __device__ __forceinline__ constexpr int row_of(int l, int x) {
     return x * 8 + l;
 }
 
-// PT: results times the pass twiddle, any u64 of their class (scratch for a next pass);
-// else canonical results.
-template <int LR1, int LR2, bool LF, bool PT>
-__global__ void __launch_bounds__(Shape<LR1, LR2>::T, LR1 == 4 && LR2 == 4 ? 2 : 1) ntt_tc_kernel(TcPass a) {
-  using S = Shape<LR1, LR2>;
+template <int LR1, int LR2, bool LF, int PT>
+__global__ void __launch_bounds__(Shape<LR1, LR2, PT>::T, LR1 == 4 && LR2 == 4 ? 2 : 1) ntt_tc_kernel(TcPass a) {
+  using S = Shape<LR1, LR2, PT>;
   constexpr int R1 = S::R1, R2 = S::R2, L = S::L, PARTS = S::PARTS, OUT = S::OUT;
   constexpr int NE = R2 / PARTS;  // input elements a thread loads
   extern __shared__ char raw[];
@@ -283,7 +286,8 @@ __global__ void __launch_bounds__(Shape<LR1, LR2>::T, LR1 == 4 && LR2 == 4 ? 2 :
   char* b2 = base;
   char* b1 = b2 + S::B2_BYTES;
   uint64_t* tw = (uint64_t*)(b1 + S::B1_BYTES);
-  char* a_all = (char*)tw + S::T_BYTES;
+  uint64_t* tw_lane = tw + kRows * R1;  // (PT = 2)
+  char* a_all = (char*)tw + S::TW_BYTES;
   char* tail = a_all + S::GROUPS * S::A_BYTES;
   uint32_t* tmem_slot = (uint32_t*)tail;
   volatile int* abort = (volatile int*)(tail + 4);
@@ -323,17 +327,24 @@ __global__ void __launch_bounds__(Shape<LR1, LR2>::T, LR1 == 4 && LR2 == 4 ? 2 :
       at_u + (m1 >> 4) * (kRows * 128) + r0 * 128 + (m1 & 1) * 8 + ((((m1 & 15) >> 1) ^ (r0 & 7)) << 4);
   // input elements m2 = 2c and 2c + 1, c = part + PARTS i, go to 16-byte chunk c of this thread's row
   const uint32_t ld_u = at_u + row * 128 + ((part ^ (row & 7)) << 4);
-  const char* in_t = at(at(a.in, m1, a.in_mb), 2 * part, a.in_step);
+  // (block layouts only with lanes together)
+  const char* in_t = LF ? at(at(a.in, m1 >> a.in_blog, a.in_hb), m1 & ((1u << a.in_blog) - 1), a.in_mb)
+                        : at(a.in, m1, a.in_mb);
+  in_t = at(in_t, 2 * part, a.in_step);
   char* out_t = at(at(a.out, x2, a.out_xb), i0, a.out_step);
-  const uint64_t* tw_t = tw + i0 * R1 + m1;
+  constexpr int TS = PT == 2 ? kRows : R1;  // stride of the first-stage twiddles
+  const uint64_t* tw_t = tw + i0 * TS + (PT == 2 ? row : m1);
 
-  // Tiles (chunk q, column y, lane group g; g fastest) go in pairs of neighbours, one to
-  // each group. A CTA has a contiguous range of pairs (few changes of chunk), or every
-  // gridDim-th pair (CTAs that run together touch neighbouring lanes together).
+  // Tiles (chunk q, column y, lane group g) go in pairs, one to each group.
+  // PT = 2: a unit is a chunk, a lane group and a range of columns; a CTA takes every
+  // gridDim-th unit (CTAs that run together touch neighbouring lanes together) and its pairs
+  // are neighbouring columns. Otherwise a unit is a chunk, pairs run over lane groups, then
+  // columns, and a CTA has a contiguous range of pairs (few changes of chunk) or every
+  // gridDim-th pair.
   const uint32_t lgroups = a.lgroups, per_q = a.lgroups * a.n_y, pairs_q = (per_q + 1) / 2;
-  const uint32_t pairs = pairs_q * a.n_q;
+  const uint32_t pairs = PT == 2 ? a.n_q * lgroups * a.y_parts : pairs_q * a.n_q;
   uint32_t pair, pair_end, step;
-  if (a.strided) {
+  if (PT == 2 || a.strided) {
     pair = blockIdx.x;
     pair_end = pairs;
     step = gridDim.x;
@@ -342,16 +353,18 @@ __global__ void __launch_bounds__(Shape<LR1, LR2>::T, LR1 == 4 && LR2 == 4 ? 2 :
     pair_end = (uint32_t)((uint64_t)pairs * (blockIdx.x + 1) / gridDim.x);
     step = 1;
   }
-  const uint32_t gstep = S::GROUPS * step, gstep_y = gstep / lgroups, gstep_g = gstep % lgroups;
+  const uint32_t gstep = PT == 2 ? S::GROUPS : S::GROUPS * step;
+  const uint32_t gstep_y = PT == 2 ? S::GROUPS : gstep / lgroups, gstep_g = PT == 2 ? 0 : gstep % lgroups;
   uint32_t phase = 0, tab_phase = 0;
-  bool loaded = false;
+  uint32_t q_loaded = ~0u;
   uint64_t x[NE];
 
   // Lanes past the last are done as copies of the last one (same loads, same stores).
   const uint32_t last_lane = a.n_lanes - 1, c8 = a.c8, c16 = a.c16;
   auto load_tile = [&](uint32_t y, uint32_t g) {
     const uint32_t lane = min(g * L + l, last_lane);
-    const char* src = at(at(in_t, y, a.in_colb), lane, a.in_laneb);
+    const char* src = at(in_t, y, a.in_colb);
+    src = LF ? at(at(src, g, a.in_gb), lane - g * L, a.in_laneb) : at(src, lane, a.in_laneb);
     if (!a.masked) {
 #pragma unroll
       for (int i = 0; i < NE; ++i) {
@@ -376,27 +389,61 @@ __global__ void __launch_bounds__(Shape<LR1, LR2>::T, LR1 == 4 && LR2 == 4 ? 2 :
   };
 
   while (pair < pair_end) {
-    const uint32_t q = pair / pairs_q, p0 = q * pairs_q;
-    const uint32_t p_end = p0 + pairs_q < pair_end ? p0 + pairs_q : pair_end;
+    uint32_t q, it, it_end, y, g;
+    if constexpr (PT == 2) {
+      const uint32_t per = lgroups * a.y_parts, r = pair % per;
+      q = pair / per;
+      g = r % lgroups;
+      y = r / lgroups * a.y_len;
+      it_end = min(y + a.y_len, a.n_y);
+      it = y += grp;
+      pair += step;
+    } else {
+      q = pair / pairs_q;
+      const uint32_t p0 = q * pairs_q, p_end = min(p0 + pairs_q, pair_end);
+      it = 2 * (pair - p0) + grp;  // within the chunk
+      it_end = min(2 * (p_end - p0), per_q);
+      y = it / lgroups;
+      g = it % lgroups;
+      pair += (p_end - pair + step - 1) / step * step;
+    }
     // the chunk's first-stage matrix and twiddles (and once the second-stage matrix)
-    if (loaded) {
+    if (q_loaded != ~0u) {
       fence_async_smem();
       __syncthreads();
     }
-    if (t == 0) {
-      const char* src = a.tab + S::B2_BYTES + (uint64_t)q * S::Q_BYTES;
-      mbar_expect(tab_bar, S::Q_BYTES + (loaded ? 0 : S::B2_BYTES));
-      if (!loaded) bulk_load(b2_u, a.tab, S::B2_BYTES, tab_bar);
-      bulk_load(b1_u, src, S::Q_BYTES, tab_bar);
+    const char* q_tab = a.tab + S::B2_BYTES + (uint64_t)q * S::Q_BYTES;
+    if (q != q_loaded) {
+      if (t == 0) {
+        const uint32_t bytes = PT == 2 ? S::B1_BYTES : S::Q_BYTES;
+        mbar_expect(tab_bar, bytes + (q_loaded == ~0u ? S::B2_BYTES : 0));
+        if (q_loaded == ~0u) bulk_load(b2_u, a.tab, S::B2_BYTES, tab_bar);
+        bulk_load(b1_u, q_tab, bytes, tab_bar);
+      }
     }
-    loaded = true;
-    char* out_q = out_t + q * a.out_q * 8;
-    uint32_t it = 2 * (pair - p0) + grp;  // within the chunk
-    const uint32_t it_end = min(2 * (p_end - p0), per_q);
-    uint32_t y = it / lgroups, g = it % lgroups;
     if (it < it_end) load_tile(y, g);
-    mbar_wait(tab_bar, tab_phase, abort, a.fail);
-    tab_phase ^= 1;
+    if constexpr (PT == 2) {
+      // w_EM^(j' m1) w_N^(j' lane) g^(m1 + lane) of every row, and w_N^(S i1 lane)
+      const uint64_t* q_tw = (const uint64_t*)(q_tab + S::B1_BYTES);
+      for (int e = t; e < kRows * R1; e += S::T) {
+        const int r = e % kRows, xx = e / kRows;
+        int ll, mm;
+        row_split<L, R1, LF>(r, &ll, &mm);
+        const uint64_t lane = (uint64_t)g * L + ll, j = (uint64_t)q * a.jq + (uint64_t)xx * a.jx;
+        uint64_t v = gl::mul(__ldg(q_tw + xx * R1 + mm), tw_pow(a.tw_lo, a.tw_hi, j * lane, a.pt_log));
+        if (a.pre.active()) v = gl::mul(v, pow_at(a.pre, lane * a.flat_lane));
+        tw[e] = v;
+      }
+      for (int e = t; e < L * R1; e += S::T)
+        tw_lane[e] = tw_pow(a.tw_lo, a.tw_hi, ((uint64_t)(e / L) * ((uint64_t)g * L + e % L)) << a.log_s, a.pt_log);
+      __syncthreads();
+    }
+    if (q != q_loaded) {
+      mbar_wait(tab_bar, tab_phase, abort, a.fail);
+      tab_phase ^= 1;
+      q_loaded = q;
+    }
+    char* out_q = out_t + q * a.out_q * 8;
     for (; it < it_end; it += gstep) {
       // operand A of the first stage
 #pragma unroll
@@ -410,10 +457,11 @@ __global__ void __launch_bounds__(Shape<LR1, LR2>::T, LR1 == 4 && LR2 == 4 ? 2 :
       bar_group(1 + grp, S::GT);
       if (gw == 0) issue<R2 / 4, 8 * R1>(tmem, at_u, b1_u, bar);
       const uint32_t lane = min(g * L + l2, last_lane);
-      char* o = at(at(out_q, y, a.out_colb), lane, a.out_laneb);
+      char* o = at(out_q, y, a.out_colb);
+      o = LF ? at(at(o, g, a.out_gb), lane - g * L, a.out_laneb) : at(o, lane, a.out_laneb);
       y += gstep_y;
       g += gstep_g;
-      if (g >= lgroups) {
+      if (PT != 2 && g >= lgroups) {
         g -= lgroups;
         ++y;
       }
@@ -427,7 +475,7 @@ __global__ void __launch_bounds__(Shape<LR1, LR2>::T, LR1 == 4 && LR2 == 4 ? 2 :
         tmem_load32(tmem_row + 32 * k, d);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const uint64_t v = mul_lazy(join_digits(d + 8 * u, c8, c16), tw_t[(4 * k + u) * R1]);
+          const uint64_t v = mul_lazy(join_digits(d + 8 * u, c8, c16), tw_t[(4 * k + u) * TS]);
           // row_of(l, i0 + x) = row_of(l, i0) + row_of(0, x), low three bits without carries
           const int ro = row_of<L, R1, LF>(0, 4 * k + u);
           const uint32_t p = (st_u ^ ((ro & 7) << 4)) + ro * 128;
@@ -439,7 +487,7 @@ __global__ void __launch_bounds__(Shape<LR1, LR2>::T, LR1 == 4 && LR2 == 4 ? 2 :
       bar_group(1 + grp, S::GT);
       if (gw == 0) issue<R1 / 4, 8 * R1>(tmem, at_u, b2_u, bar);
       uint64_t f = 0, rho = 0;
-      if constexpr (PT) {  // w_N^((j' + S i1) lane) g^lane as a geometric sequence in i1
+      if constexpr (PT == 1) {  // w_N^((j' + S i1) lane) g^lane as a geometric sequence in i1
         rho = tw_pow(a.tw_lo, a.tw_hi, (uint64_t)lane << a.log_s, a.pt_log);
         const uint64_t j = (uint64_t)q * a.jq + (uint64_t)x2 * a.jx + ((uint64_t)i0 << a.log_s);
         f = tw_pow(a.tw_lo, a.tw_hi, j * lane, a.pt_log);
@@ -454,16 +502,16 @@ __global__ void __launch_bounds__(Shape<LR1, LR2>::T, LR1 == 4 && LR2 == 4 ? 2 :
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           uint64_t v = join_digits(d + 8 * u, c8, c16);
-          if constexpr (PT) {
+          if constexpr (PT == 1) {
             v = mul_lazy(v, f);
             f = mul_lazy(f, rho);
           }
-          if (!PT || a.canon) v = canonical(v);
+          if constexpr (PT == 2) v = mul_lazy(v, tw_lane[(i0 + 4 * k + u) * L + l2]);
+          if (PT == 0 || a.canon) v = canonical(v);
           *(uint64_t*)at(o, 4 * k + u, a.out_step) = v;
         }
       }
     }
-    pair += (p_end - pair + step - 1) / step * step;
   }
   tc_fence_before();
   __syncthreads();
@@ -473,37 +521,68 @@ __global__ void __launch_bounds__(Shape<LR1, LR2>::T, LR1 == 4 && LR2 == 4 ? 2 :
   }
 }
 
-template <int LR1, int LR2, bool LF, bool PT>
+template <int LR1, int LR2, bool LF, int PT>
 cudaError_t launch(TcPass a, cudaStream_t s) {
-  using S = Shape<LR1, LR2>;
+  using S = Shape<LR1, LR2, PT>;
   auto kern = ntt_tc_kernel<LR1, LR2, LF, PT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
   if (e != cudaSuccess) return e;
-  const uint64_t lgroups = (a.n_lanes + S::L - 1) / S::L, pairs = (lgroups * a.n_y + 1) / 2 * a.n_q;
+  const uint64_t lgroups = (a.n_lanes + S::L - 1) / S::L, fit = 148 * (LR1 == 4 && LR2 == 4 ? 2 : 1);
+  const uint64_t in_m2 = a.in_block ? S::R1 / a.in_block * a.in_h : S::R1 * a.in_m;
+  const uint64_t in_g = a.in_g ? a.in_g : S::L * a.in_lane, out_g = a.out_g ? a.out_g : S::L * a.out_lane;
   // the kernel's strides are 32-bit byte counts
-  const uint64_t strides[] = {a.in_m * S::R1, a.in_lane, a.in_col, a.out_i, a.out_x, a.out_lane, a.out_col};
+  const uint64_t strides[] = {in_m2, in_g, a.in_col, a.in_h, a.out_i, a.out_x, out_g, a.out_col};
   for (uint64_t v : strides)
     if (v >= 1ull << 29) return cudaErrorInvalidValue;
-  if (pairs >= 1ull << 30) return cudaErrorInvalidValue;
+  a.lgroups = (uint32_t)lgroups;
+  a.in_blog = 31;
+  if (a.in_block)
+    for (a.in_blog = 0; (1u << a.in_blog) < a.in_block;) ++a.in_blog;
   a.in_mb = (uint32_t)(a.in_m * 8);
+  a.in_hb = (uint32_t)(a.in_h * 8);
+  a.in_step = (uint32_t)(in_m2 * 8);
   a.in_laneb = (uint32_t)(a.in_lane * 8);
+  a.in_gb = (uint32_t)(in_g * 8);
   a.in_colb = (uint32_t)(a.in_col * 8);
   a.out_xb = (uint32_t)(a.out_x * 8);
-  a.out_laneb = (uint32_t)(a.out_lane * 8);
-  a.out_colb = (uint32_t)(a.out_col * 8);
-  a.lgroups = (uint32_t)lgroups;
-  a.in_step = (uint32_t)(a.in_m * S::R1 * 8);
   a.out_step = (uint32_t)(a.out_i * 8);
+  a.out_laneb = (uint32_t)(a.out_lane * 8);
+  a.out_gb = (uint32_t)(out_g * 8);
+  a.out_colb = (uint32_t)(a.out_col * 8);
   a.masked = a.in_valid <= (a.n_lanes - 1) * a.flat_lane + (uint64_t)(S::R1 * S::R2 - 1) * a.flat_m;
   a.c8 = 1u << 8;
   a.c16 = 1u << 16;
-  const uint64_t fit = 148 * (LR1 == 4 && LR2 == 4 ? 2 : 1);
-  // a CTA takes up to 24 pairs, so that CTAs of a higher-priority stream get in between
-  const uint64_t most = (pairs + 23) / 24;
-  const uint64_t grid = pairs <= fit ? pairs : (most + fit - 1) / fit * fit;
+  // a CTA takes up to 24 pairs of tiles (about 100 us), so that CTAs of a higher-priority
+  // stream get in between
+  uint64_t units, pairs;
+  if (PT == 2) {
+    // column ranges of at least 8 columns, as many as it takes to fill whole waves of CTAs
+    uint32_t parts = 1;
+    while ((a.n_y + 2 * parts - 1) / (2 * parts) >= 8 && parts < 16) {
+      const uint64_t u = lgroups * a.n_q * parts;
+      if (u * 100 >= (u + fit - 1) / fit * fit * 93) break;
+      parts *= 2;
+    }
+    a.y_len = (a.n_y + parts - 1) / parts;
+    a.y_parts = (a.n_y + a.y_len - 1) / a.y_len;
+    units = lgroups * a.n_q * a.y_parts;
+    pairs = units * ((a.y_len + 1) / 2);
+  } else {
+    units = pairs = (lgroups * a.n_y + 1) / 2 * a.n_q;
+  }
+  if (pairs >= 1ull << 30 || lgroups * a.n_y >= 1ull << 30) return cudaErrorInvalidValue;
+  const uint64_t waves = (pairs + 24 * fit - 1) / (24 * fit);
+  const uint64_t grid = std::min(units, waves * fit);
   SG_LAUNCH_SCOPE("ntt_pass", s);
-  kern<<<(unsigned)std::min(grid, pairs), S::T, S::SMEM, s>>>(a);
+  kern<<<(unsigned)grid, S::T, S::SMEM, s>>>(a);
   return cudaGetLastError();
+}
+
+template <int LR1, int LR2>
+cudaError_t launch_mode(const TcPass& a, bool lanes_fast, int pt, cudaStream_t s) {
+  if (pt == 1) return launch<LR1, LR2, true, 1>(a, s);
+  if (pt == 2) return launch<LR1, LR2, true, 2>(a, s);
+  return lanes_fast ? launch<LR1, LR2, true, 0>(a, s) : launch<LR1, LR2, false, 0>(a, s);
 }
 
 // ------------------------------------------------------------------ tables
@@ -552,6 +631,8 @@ uint64_t image_bytes(int lr1, int lr2, uint32_t n_q) {
 }
 
 }  // namespace
+
+int ntt_tc_lanes(int log_m) { return log_m == 10 ? 4 : 8; }
 
 bool ntt_tc_ok(int log_m) { return log_m >= 8 && log_m <= 10; }
 
@@ -691,17 +772,16 @@ cudaError_t ntt_tc_pass(const TcPass& a, bool lanes_fast, cudaStream_t s) {
     ntt_tc_drop(a, s);
     return cudaSuccess;
   }
-  const bool pt = a.pt_log > 0;
+  // The lane tables of PT = 2 cost about as much as a pair of tiles, so they are shared by at
+  // least 8 columns, and there have to be two waves of such units (6 x 2^20: 138 us with
+  // them, 128 without; 100 x 2^14: 67 and 51; 64 x 2^20: 934 and 979).
+  const uint64_t units = (uint64_t)(a.n_lanes / ntt_tc_lanes(a.log_m)) * a.n_q * (a.n_y / 8);
+  const int pt = a.pt_log == 0 ? 0 : units < 2 * 148 * (a.log_m == 8 ? 2 : 1) ? 1 : 2;
   cudaError_t e = cudaErrorInvalidValue;
   if (!pt || lanes_fast) switch (a.log_m) {
-      case 8:
-        e = pt ? launch<4, 4, true, true>(a, s) : lanes_fast ? launch<4, 4, true, false>(a, s) : launch<4, 4, false, false>(a, s);
-        break;
-      case 9:
-        e = pt ? launch<4, 5, true, true>(a, s) : lanes_fast ? launch<4, 5, true, false>(a, s) : launch<4, 5, false, false>(a, s);
-        break;
-      default:
-        e = pt ? launch<5, 5, true, true>(a, s) : lanes_fast ? launch<5, 5, true, false>(a, s) : launch<5, 5, false, false>(a, s);
+      case 8: e = launch_mode<4, 4>(a, lanes_fast, pt, s); break;
+      case 9: e = launch_mode<4, 5>(a, lanes_fast, pt, s); break;
+      default: e = launch_mode<5, 5>(a, lanes_fast, pt, s);
     }
   ntt_tc_drop(a, s);
   return e;

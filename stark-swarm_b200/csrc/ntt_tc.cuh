@@ -19,6 +19,10 @@ struct TcPass {
   const uint64_t* in;
   uint64_t* out;
   uint64_t in_col, out_col, in_lane, in_m, out_lane, out_q, out_x, out_i;
+  // optional layouts in blocks: lane groups (a tile's lanes, ntt_tc_lanes) at their own stride, and
+  // input points m at m / in_block * in_h + m % in_block * in_m
+  uint64_t in_g, out_g, in_h;
+  uint32_t in_block;
   uint32_t n_lanes, n_y, n_q, jq, jx;
   uint64_t flat_m, flat_lane, in_valid;
   int log_m, log_s, pt_log;
@@ -30,11 +34,13 @@ struct TcPass {
   const char* tab;
   const uint64_t *tw_lo, *tw_hi;
   int* fail;
-  uint32_t lgroups, in_step, in_mb, in_laneb, in_colb, out_step, out_xb, out_laneb, out_colb, c8, c16;
+  uint32_t lgroups, y_parts, y_len, in_blog, in_step, in_mb, in_hb, in_laneb, in_gb, in_colb;
+  uint32_t out_step, out_xb, out_laneb, out_gb, out_colb, c8, c16;
   bool masked, own_tab;
 };
 
 bool ntt_tc_ok(int log_m);
+int ntt_tc_lanes(int log_m);  // lanes of a tile
 // the fields that follow from M = 2^log_m and E = 2^log_e (chunks of adjacent j'); the caller sets the rest
 TcPass ntt_tc_args(int log_m, int log_e);
 // The pass's byte matrices and twiddles (from pre, scale, flat_m, jq, jx and the shape), in

@@ -95,6 +95,12 @@ bool lde_by_cosets(uint64_t n_trace, uint64_t blowup) {
 void lde_core(sg_ctx* c, const uint64_t* d_trace, uint64_t w, uint64_t n_trace, uint64_t blowup,
               const ShiftTables& sh, uint64_t* coef, uint64_t* scratch, uint64_t* d_out) {
   const uint64_t n0 = n_trace * blowup;
+  const cudaError_t e = ntt_lde(c->tw, d_trace, coef, d_out, (uint32_t)w, (int)log2_exact(n_trace),
+                                (int)log2_exact(blowup), scratch, c->stream, sh.active ? &sh.spec : nullptr);
+  if (e != cudaErrorNotSupported) {
+    cuda_check(e, "lde");
+    return;
+  }
   ntt(c, d_trace, coef, (uint32_t)w, n_trace, n_trace, log2_exact(n_trace), true, n_trace, scratch);
   if (lde_by_cosets(n_trace, blowup)) {
     cuda_check(ntt_coset_eval(c->tw, coef, d_out, (uint32_t)w, (int)log2_exact(n_trace), (int)log2_exact(blowup),

@@ -55,6 +55,25 @@ def test_lde(ctx, w, log_n, blowup, shift):
     assert np.array_equal(ctx.lde(tr, blowup, shift), O.lde(tr, blowup, shift))
 
 
+# enough columns for the first pass's lane tables (whole waves of units of 8 columns and
+# more, a ragged last range), and the LDE with its coefficients in blocks
+@pytest.mark.parametrize("cols,log_n", [(50, 16), (37, 17), (33, 18), (24, 20)])
+def test_many_columns(ctx, cols, log_n):
+    rng = np.random.default_rng(cols)
+    x = field(rng, cols, 1 << log_n)
+    got = ctx.ntt(x, log_n, True)
+    for c in range(0, cols, 5):
+        assert np.array_equal(got[c], O.ntt(x[c], True)), c
+
+
+@pytest.mark.parametrize("w,log_n,blowup,shift", [(20, 16, 8, 7), (9, 17, 4, 1), (35, 18, 2, 3), (3, 19, 4, 7), (2, 20, 8, 7)])
+def test_lde_blocked_coefficients(ctx, w, log_n, blowup, shift):
+    rng = np.random.default_rng(w)
+    tr = field(rng, w, 1 << log_n)
+    got, pick = ctx.lde(tr, blowup, shift), [0, w // 2, w - 1]
+    assert np.array_equal(got[pick], O.lde(np.ascontiguousarray(tr[pick]), blowup, shift))
+
+
 def test_repeated_calls_and_tables(ctx):
     """A shape's tables are built once and shared by later calls, another shift in between."""
     rng = np.random.default_rng(5)
