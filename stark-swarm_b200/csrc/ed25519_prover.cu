@@ -270,7 +270,9 @@ void merge_cosets_on_device(sg_ctx* c, const ed25519::Witness& w, const EdShape&
   cuda_check(ntt_batch(c->tw, d_trace, coef.p, (uint32_t)W, n_trace, n_trace, (int)lt, true, n_trace, scratch.p, s),
              "ed25519 trace intt");
   for (uint64_t r0 = 0; r0 < blowup; r0 += G) {
-    for (uint64_t g = 0; g < G; ++g) {
+    const cudaError_t e = ntt_cosets(c->tw, coef.p, ev.p, (uint32_t)W, (int)lt, (int)(ln - lt), (uint32_t)r0, (uint32_t)G, s);
+    if (e != cudaErrorNotSupported) cuda_check(e, "ed25519 cosets");
+    for (uint64_t g = 0; e == cudaErrorNotSupported && g < G; ++g) {
       const uint64_t r = r0 + g;
       PowSpec twist;
       if (r > 0) {

@@ -772,6 +772,29 @@ cudaError_t ntt_coset_eval(const NttTables& t, const uint64_t* coef, uint64_t* o
   return launch_pass_dyn(log_m, a, false, n_cols, s);
 }
 
+cudaError_t ntt_cosets(const NttTables& t, const uint64_t* coef, uint64_t* out, uint32_t n_cols, int log_m, int log_b,
+                       uint32_t r0, uint32_t g, cudaStream_t s) {
+  // a coset is one chunk where both stages have the same radix
+  if ((log_m != 8 && log_m != 10) || log_m + log_b > kMaxLogN || r0 + g > (1u << log_b)) return cudaErrorNotSupported;
+  const uint64_t M = 1ull << log_m;
+  TcPass p = ntt_tc_args(log_m, log_b);
+  p.in = coef;
+  p.out = out;
+  p.n_q = g;
+  p.j0 = r0;
+  p.jq = 1;
+  p.jx = 1u << log_b;
+  p.in_lane = M;
+  p.in_m = 1;
+  p.out_lane = g * M;
+  p.out_q = M;
+  p.out_x = 1;
+  p.out_i = 1ull << (log_m / 2);
+  p.n_lanes = n_cols;
+  p.in_valid = M;
+  return ntt_tc_tables(t, &p, false, s) ? ntt_tc_pass(p, false, s) : cudaErrorNotSupported;
+}
+
 cudaError_t pow_table_device(const NttTables& t, uint64_t mult, int log_n, uint64_t len, uint64_t* tab,
                              cudaStream_t s) {
   if (len == 0) return cudaSuccess;

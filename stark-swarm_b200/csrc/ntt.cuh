@@ -104,6 +104,13 @@ bool ntt_coset_eval_ok(int log_m, int log_b);
 cudaError_t ntt_coset_eval(const NttTables& t, const uint64_t* coef, uint64_t* out, uint32_t n_cols, int log_m,
                            int log_b, cudaStream_t s, const PowSpec* pre = nullptr);
 
+// The values of the same polynomials on the cosets r0 .. r0 + g - 1 of those N points (point
+// i of coset r is w_N^(r + 2^log_b i)), coset by coset: column c's coset r0 + q at
+// out + (c g + q) M. cudaErrorNotSupported (nothing done) unless M is 2^8 or 2^10 and the
+// transform runs on the tensor cores.
+cudaError_t ntt_cosets(const NttTables& t, const uint64_t* coef, uint64_t* out, uint32_t n_cols, int log_m, int log_b,
+                       uint32_t r0, uint32_t g, cudaStream_t s);
+
 // Forward transform of w zero-padded columns (as ntt_batch with in_stride and
 // n_valid) whose last pass, a 2^7-point DFT, hashes the rows of the result into
 // Merkle leaves instead of storing them: leaf r (kc::kDigestLanes lanes at

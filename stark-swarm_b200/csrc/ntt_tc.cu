@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(Shape<LR1, LR2, PT>::T, LR1 == 4 && LR2 == 4 ?
         const int r = e % kRows, xx = e / kRows;
         int ll, mm;
         row_split<L, R1, LF>(r, &ll, &mm);
-        const uint64_t lane = (uint64_t)g * L + ll, j = (uint64_t)q * a.jq + (uint64_t)xx * a.jx;
+        const uint64_t lane = (uint64_t)g * L + ll, j = a.j0 + (uint64_t)q * a.jq + (uint64_t)xx * a.jx;
         uint64_t v = gl::mul(__ldg(q_tw + xx * R1 + mm), tw_pow(a.tw_lo, a.tw_hi, j * lane, a.pt_log));
         if (a.pre.active()) v = gl::mul(v, pow_at(a.pre, lane * a.flat_lane));
         tw[e] = v;
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(Shape<LR1, LR2, PT>::T, LR1 == 4 && LR2 == 4 ?
       uint64_t f = 0, rho = 0;
       if constexpr (PT == 1) {  // w_N^((j' + S i1) lane) g^lane as a geometric sequence in i1
         rho = tw_pow(a.tw_lo, a.tw_hi, (uint64_t)lane << a.log_s, a.pt_log);
-        const uint64_t j = (uint64_t)q * a.jq + (uint64_t)x2 * a.jx + ((uint64_t)i0 << a.log_s);
+        const uint64_t j = a.j0 + (uint64_t)q * a.jq + (uint64_t)x2 * a.jx + ((uint64_t)i0 << a.log_s);
         f = tw_pow(a.tw_lo, a.tw_hi, j * lane, a.pt_log);
         if (a.pre.active()) f = gl::mul(f, pow_at(a.pre, (uint64_t)lane * a.flat_lane));
       }
@@ -592,7 +592,7 @@ cudaError_t launch_mode(const TcPass& a, bool lanes_fast, int pt, cudaStream_t s
 struct PrepArgs {
   char* out;
   int lr1, lr2, log_s;
-  uint32_t n_q, jq, jx;
+  uint32_t n_q, j0, jq, jx;
   uint64_t flat_m, scale;
   PowSpec pre;
   const uint64_t *lo, *hi;
@@ -612,13 +612,13 @@ __global__ void __launch_bounds__(256) tc_prep_kernel(PrepArgs a) {
     char* o = a.out + 64 * n2 + q * q_bytes;
     if (r < n1) {
       const int m = (int)(r & (R2 - 1)), x = (int)(r >> a.lr2);
-      uint64_t v = tw_pow(a.lo, a.hi, (q * a.jq + (uint64_t)x * a.jx) * m, a.log_s);
+      uint64_t v = tw_pow(a.lo, a.hi, (a.j0 + q * a.jq + (uint64_t)x * a.jx) * m, a.log_s);
       if (a.pre.active()) v = gl::mul(v, pow_at(a.pre, ((uint64_t)m << a.lr1) * a.flat_m));
       if (a.scale != 1) v = gl::mul(v, a.scale);
       store_digits(o, 8 * R1, x, m, v);
     } else {
       const int m = (int)((r - n1) & (R1 - 1)), x = (int)((r - n1) >> a.lr1);
-      uint64_t v = tw_pow(a.lo, a.hi, (q * a.jq + (uint64_t)x * a.jx) * m, a.log_s + a.lr1);
+      uint64_t v = tw_pow(a.lo, a.hi, (a.j0 + q * a.jq + (uint64_t)x * a.jx) * m, a.log_s + a.lr1);
       if (a.pre.active()) v = gl::mul(v, pow_at(a.pre, (uint64_t)m * a.flat_m));
       ((uint64_t*)(o + 64 * n1))[x * R1 + m] = v;
     }
@@ -662,7 +662,7 @@ struct TcCache {
     bool done = false;
   };
   std::mutex mu;
-  std::map<std::tuple<int, int, uint32_t, uint32_t, bool, uint64_t>, Entry> map;
+  std::map<std::tuple<int, int, uint32_t, uint32_t, uint32_t, uint32_t, bool, uint64_t>, Entry> map;
   uint64_t bytes = 0;
 };
 TcCache* tc_cache_new() { return new (std::nothrow) TcCache; }
@@ -677,7 +677,7 @@ void tc_cache_free(TcCache* c) {
 
 static cudaError_t build(const NttTables& t, const TcPass& a, bool inverse, char* d, cudaStream_t s) {
   const int lr1 = a.log_m == 10 ? 5 : 4, lr2 = a.log_m - lr1;
-  PrepArgs p{d, lr1, lr2, a.log_s, a.n_q, a.jq, a.jx, a.flat_m, a.scale, a.pre,
+  PrepArgs p{d, lr1, lr2, a.log_s, a.n_q, a.j0, a.jq, a.jx, a.flat_m, a.scale, a.pre,
              inverse ? t.d_inv_lo : t.d_fwd_lo, inverse ? t.d_inv_hi : t.d_fwd_hi};
   const uint64_t total = (1ull << (2 * lr1)) + a.n_q * ((1ull << (2 * lr1)) + (1ull << a.log_m));
   SG_LAUNCH_SCOPE("ntt_tables", s);
@@ -696,7 +696,7 @@ bool ntt_tc_tables(const NttTables& t, TcPass* a, bool inverse, cudaStream_t s) 
   a->fail = ntt_tc_fail_flag();
   if (!a->pre.active()) {
     std::lock_guard<std::mutex> g(t.tc->mu);
-    const auto key = std::make_tuple(a->log_m, a->log_s, a->jq, a->jx, inverse, a->scale);
+    const auto key = std::make_tuple(a->log_m, a->log_s, a->n_q, a->j0, a->jq, a->jx, inverse, a->scale);
     auto it = t.tc->map.find(key);
     if (it != t.tc->map.end()) {
       TcCache::Entry& e = it->second;

@@ -9,7 +9,7 @@ namespace sg {
 
 // n_y outer columns of n_lanes independent transforms of M = R1 R2 points, each giving
 // E M outputs j = j' + S i1 (S = E R2 = 2^log_s, i1 < R1) in n_q chunks of R1 values of j':
-// j' = q jq + x jx. R1 = 16 for M = 2^8 and 2^9, 32 for 2^10.
+// j' = j0 + q jq + x jx (adjacent ones, or with jx = E a coset's). R1 = 16 for M = 2^8 and 2^9, 32 for 2^10.
 //   input  (y, lane, m):      in + y in_col + lane in_lane + m in_m
 //   output (y, lane, q, x, i1): out + y out_col + lane out_lane + q out_q + x out_x + i1 out_i
 // Inputs at flat index m flat_m + lane flat_lane >= in_valid are zero; pre multiplies
@@ -23,7 +23,7 @@ struct TcPass {
   // input points m at m / in_block * in_h + m % in_block * in_m
   uint64_t in_g, out_g, in_h;
   uint32_t in_block;
-  uint32_t n_lanes, n_y, n_q, jq, jx;
+  uint32_t n_lanes, n_y, n_q, j0, jq, jx;
   uint64_t flat_m, flat_lane, in_valid;
   int log_m, log_s, pt_log;
   uint64_t scale;

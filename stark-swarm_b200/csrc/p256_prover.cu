@@ -128,7 +128,9 @@ void p256_merge_cosets(sg_ctx* c, const uint64_t* d_trace, uint64_t n_trace, uin
              "p256 trace intt");
   for (uint64_t r0 = 0; r0 < blowup; r0 += G) {
     // column col of coset r0 + g at ev[col * G n_trace + g n_trace]
-    for (uint64_t g = 0; g < G; ++g) {
+    const cudaError_t e = ntt_cosets(c->tw, coef.p, ev.p, (uint32_t)W, (int)lt, (int)(ln - lt), (uint32_t)r0, (uint32_t)G, s);
+    if (e != cudaErrorNotSupported) cuda_check(e, "p256 cosets");
+    for (uint64_t g = 0; e == cudaErrorNotSupported && g < G; ++g) {
       const uint64_t r = r0 + g;
       PowSpec twist;
       if (r > 0) {
