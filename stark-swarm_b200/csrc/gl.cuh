@@ -180,6 +180,13 @@ struct Acc128 {
     asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\taddc.cc.u32 %2, %2, %6;\n\taddc.u32 %3, %3, 0;"
         : "+r"(a0), "+r"(a1), "+r"(a2), "+r"(a3) : "r"(y0), "r"(y1), "r"(y2));
   }
+  // the same for an f that is not known at compile time
+  __device__ __forceinline__ void add_shl_var(uint64_t x, unsigned f) {
+    const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32);
+    asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\taddc.cc.u32 %2, %2, %6;\n\taddc.u32 %3, %3, 0;"
+        : "+r"(a0), "+r"(a1), "+r"(a2), "+r"(a3)
+        : "r"(x0 << f), "r"(__funnelshift_l(x0, x1, f)), "r"(__funnelshift_l(x1, 0, f)));
+  }
   // x 2^(32 + f), f < 32: the same three words one limb up (the sum must stay below 2^128)
   __device__ __forceinline__ void add_shl32(uint64_t x, unsigned f) {
     uint32_t y0, y1, y2;
@@ -197,6 +204,41 @@ struct Acc128 {
   }
   __device__ __forceinline__ uint64_t reduce() const {
     return reduce128((uint64_t)a3 << 32 | a2, (uint64_t)a1 << 32 | a0);
+  }
+};
+#endif
+#if defined(__CUDACC__)
+// a b mod p as some u64 (not always below p), for any u64 a and b: with the product's
+// words x0..x3, x0 + (x1 + x2) 2^32 - (x2 + x3); the word above 2^64 (-1, 0 or 1) comes
+// back times 2^32 - 1, which neither carries nor borrows again. 15 instructions against
+// mul's 22 (29 and 36 clocks a warp). add and sub take such a value as first operand.
+__device__ __forceinline__ uint64_t mul_any(uint64_t a, uint64_t b) {
+  const unsigned __int128 x = (unsigned __int128)a * b;
+  const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32), x2 = (uint32_t)(x >> 64), x3 = (uint32_t)(x >> 96);
+  const uint64_t lo = (uint64_t)x0 - ((uint64_t)x2 + x3);                              // signed
+  const uint64_t hi = (uint64_t)x1 + x2 + (uint64_t)((int64_t)lo >> 32);               // signed, below 2^33
+  const int64_t c = (int32_t)(hi >> 32);
+  return (hi << 32 | (uint32_t)lo) + ((uint64_t)c << 32) - (uint64_t)c;
+}
+// Sum of unreduced products a b (any u64, fewer than 2^31 of them): the products of equal
+// halves in e0..e4, the crossed ones, 32 bits up, in m0..m2; 11 instructions a term.
+struct AccProd {
+  uint32_t e0 = 0, e1 = 0, e2 = 0, e3 = 0, e4 = 0, m0 = 0, m1 = 0, m2 = 0;
+  __device__ __forceinline__ void add(uint64_t a, uint64_t b) {
+    const uint32_t a0 = (uint32_t)a, a1 = (uint32_t)(a >> 32), b0 = (uint32_t)b, b1 = (uint32_t)(b >> 32);
+    asm("mad.lo.cc.u32 %0, %5, %7, %0;\n\tmadc.hi.cc.u32 %1, %5, %7, %1;\n\t"
+        "madc.lo.cc.u32 %2, %6, %8, %2;\n\tmadc.hi.cc.u32 %3, %6, %8, %3;\n\taddc.u32 %4, %4, 0;"
+        : "+r"(e0), "+r"(e1), "+r"(e2), "+r"(e3), "+r"(e4) : "r"(a0), "r"(a1), "r"(b0), "r"(b1));
+    asm("mad.lo.cc.u32 %0, %3, %6, %0;\n\tmadc.hi.cc.u32 %1, %3, %6, %1;\n\taddc.u32 %2, %2, 0;\n\t"
+        "mad.lo.cc.u32 %0, %4, %5, %0;\n\tmadc.hi.cc.u32 %1, %4, %5, %1;\n\taddc.u32 %2, %2, 0;"
+        : "+r"(m0), "+r"(m1), "+r"(m2) : "r"(a0), "r"(a1), "r"(b0), "r"(b1));
+  }
+  // canonical; the word above 2^128 counts -2^32 each (2^96 = -1)
+  __device__ __forceinline__ uint64_t reduce() const {
+    uint32_t w1, w2, w3, w4;
+    asm("add.cc.u32 %0, %4, %5;\n\taddc.cc.u32 %1, %6, %7;\n\taddc.cc.u32 %2, %8, %9;\n\taddc.u32 %3, %10, 0;"
+        : "=&r"(w1), "=&r"(w2), "=&r"(w3), "=r"(w4) : "r"(e1), "r"(m0), "r"(e2), "r"(m1), "r"(e3), "r"(m2), "r"(e4));
+    return sub(reduce128((uint64_t)w3 << 32 | w2, (uint64_t)w1 << 32 | e0), (uint64_t)w4 << 32);
   }
 };
 #endif

@@ -39,18 +39,6 @@ namespace {
 // ------------------------------------------------------------------ lazy field arithmetic
 // Any u64 stands for its residue here; only values that leave a transform are canonical.
 
-// a b mod p as some u64, for any u64 a and b: with the product's words x0..x3,
-// x0 + (x1 + x2) 2^32 - (x2 + x3); the word above 2^64 (-1, 0 or 1) comes back times
-// 2^32 - 1, which neither carries nor borrows again.
-__device__ __forceinline__ uint64_t mul_lazy(uint64_t a, uint64_t b) {
-  const unsigned __int128 x = (unsigned __int128)a * b;
-  const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32), x2 = (uint32_t)(x >> 64), x3 = (uint32_t)(x >> 96);
-  const uint64_t lo = (uint64_t)x0 - ((uint64_t)x2 + x3);                              // signed
-  const uint64_t hi = (uint64_t)x1 + x2 + (uint64_t)((int64_t)lo >> 32);               // signed, below 2^33
-  const int64_t c = (int32_t)(hi >> 32);
-  return (hi << 32 | (uint32_t)lo) + ((uint64_t)c << 32) - (uint64_t)c;
-}
-
 // sum_d D_d 2^(8d) mod p as some u64, for D_d <= 256 * 255^2: pairs D_d + 256 D_(d+1)
 // fit 32 bits (257 * 256 * 255^2 < 2^32), the four pairs are 16 bits apart, and the
 // word above 2^64 (below 2^17) is folded once.
@@ -475,7 +463,7 @@ __global__ void __launch_bounds__(Shape<LR1, LR2, PT>::T, LR1 == 4 && LR2 == 4 ?
         tmem_load32(tmem_row + 32 * k, d);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const uint64_t v = mul_lazy(join_digits(d + 8 * u, c8, c16), tw_t[(4 * k + u) * TS]);
+          const uint64_t v = gl::mul_any(join_digits(d + 8 * u, c8, c16), tw_t[(4 * k + u) * TS]);
           // row_of(l, i0 + x) = row_of(l, i0) + row_of(0, x), low three bits without carries
           const int ro = row_of<L, R1, LF>(0, 4 * k + u);
           const uint32_t p = (st_u ^ ((ro & 7) << 4)) + ro * 128;
@@ -503,10 +491,10 @@ __global__ void __launch_bounds__(Shape<LR1, LR2, PT>::T, LR1 == 4 && LR2 == 4 ?
         for (int u = 0; u < 4; ++u) {
           uint64_t v = join_digits(d + 8 * u, c8, c16);
           if constexpr (PT == 1) {
-            v = mul_lazy(v, f);
-            f = mul_lazy(f, rho);
+            v = gl::mul_any(v, f);
+            f = gl::mul_any(f, rho);
           }
-          if constexpr (PT == 2) v = mul_lazy(v, tw_lane[(i0 + 4 * k + u) * L + l2]);
+          if constexpr (PT == 2) v = gl::mul_any(v, tw_lane[(i0 + 4 * k + u) * L + l2]);
           if (PT == 0 || a.canon) v = canonical(v);
           *(uint64_t*)at(o, 4 * k + u, a.out_step) = v;
         }

@@ -14,6 +14,7 @@
 
 #include "counters.hpp"
 #include "gl.cuh"
+#include "hash_phi.cuh"
 #include "sha256_air.cuh"
 
 namespace sg {
@@ -147,122 +148,88 @@ __global__ void __launch_bounds__(256) sha256_expand_kernel(const sha::BlockWitn
 }
 
 // ------------------------------------------------------------------ device Phi
-struct Acc {
-  const uint64_t* lam;
-  uint64_t phi;
-  uint32_t k;
-  __device__ __forceinline__ void push(uint64_t v) {
-    phi = gl::add(phi, gl::mul(__ldg(lam + k), v));
-    ++k;
-  }
-  __device__ __forceinline__ void zeros(uint32_t cnt) { k += cnt; }  // disabled slots contribute 0
+// tables indexed by the chunk: constant memory (as local arrays they would be built on the stack)
+__constant__ uint32_t kBoolBits[8] = {sha::BIT_A, sha::BIT_B, sha::BIT_C, sha::BIT_E, sha::BIT_F, sha::BIT_G, sha::BIT_WW14, sha::BIT_WW1};
+__constant__ uint32_t kBoolWord[8] = {sha::A_a, sha::A_b, sha::A_c, sha::A_e, sha::A_f, sha::A_g, sha::WW0 + 14, sha::WW0 + 1};
+struct Sg {
+  uint32_t bits, t, bit, w;
+  int r1, r2, r3;
+  bool shift;
 };
-
-__device__ __forceinline__ uint64_t xor_poly(uint64_t x, uint64_t y) {
-  // x + y - 2xy
-  return gl::sub(gl::add(x, y), gl::add(gl::mul(x, y), gl::mul(x, y)));
-}
+__constant__ Sg kSg[4] = {{sha::BIT_A, sha::S0_T, sha::S0_BIT, sha::S0_W, 2, 13, 22, false},
+                           {sha::BIT_E, sha::S1_T, sha::S1_BIT, sha::S1_W, 6, 11, 25, false},
+                           {sha::BIT_WW1, sha::SS0_T, sha::SS0_BIT, sha::SS0_W, 7, 18, 3, true},
+                           {sha::BIT_WW14, sha::SS1_T, sha::SS1_BIT, sha::SS1_W, 17, 19, 10, true}};
 
 // Point i of a column-major evaluation buffer (n points per column): cur = point
 // i, nxt = point (i + step) mod n, trace_row = i / row_div. The full LDE uses
 // (step, row_div) = (blowup, blowup); one coset of it uses (1, 1).
-// The 766 constraints are split into kPhiChunks chunks (grid.y): constraints
-// 0-263 (bit booleanity, bit -> word packs), 264-523 (the four Sigma / sigma
-// blocks) and 524-765 (Ch, Maj, carries, register shifts, H, W window,
-// schedule). Chunk c writes its part of Phi at part[c n + i]; sha256_phi_sum adds
-// them. Three shorter threads per point keep more warps in flight than one long
-// one: a thread of the unsplit kernel spent most of its time waiting on loads.
-constexpr int kPhiChunks = 3;
-__global__ void __launch_bounds__(128, 4) sha256_phi_kernel(const uint64_t* __restrict__ lde, uint64_t n, uint64_t step,
+//
+// The 766 constraints go in 16 chunks of 33 to 96, one CTA each: the eight words'
+// booleanity and packs, the four Sigma / sigma blocks, Ch, the products of Maj, the
+// xors of Maj, and the rest. Chunk c writes its part of Phi at part[c n + i];
+// sha256_phi_sum adds them. A point's chunks are neighbouring CTAs, so the bit columns
+// that several of them read come from L2. Bound by latency before (3 chunks, 128
+// registers, 16 warps an SM: 306 clocks a constraint and warp against some 110 of
+// instructions); small chunks in 64 registers keep twice the warps in flight, and the
+// unreduced sums take the reduction and the field addition out of every term. 2^17
+// points (756 columns, 0.8 GB): 852 -> 324 us; a two-block proof's 8192: 115 -> 38 us.
+constexpr int kPhiChunks = 16;
+__global__ void __launch_bounds__(128, 8) sha256_phi_kernel(const uint64_t* __restrict__ lde, uint64_t n, uint64_t step,
                                                          uint64_t row_div, uint64_t n_blocks,
                                                          const uint64_t* __restrict__ lam, uint64_t* __restrict__ part) {
   using namespace sha;
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  const uint32_t chunk = blockIdx.x % kPhiChunks;
+  const uint64_t i = (blockIdx.x / kPhiChunks) * (uint64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const uint32_t chunk = blockIdx.y;
+  const hphi::Cells C{lde + i, n};
+  uint64_t* out = part + chunk * n + i;
+  if (chunk < 8) {
+    gl::AccProd acc;
+    hphi::bool_pack(acc, C, kBoolBits[chunk], kBoolWord[chunk], lam + 32 * chunk, lam + 256 + chunk);
+    *out = acc.reduce();
+    return;
+  }
+  if (chunk < 12) {
+    // Sigma0(a), Sigma1(e) (rotations), sigma0(W[t-14]), sigma1(W[t-1]) (two rotations + a shift)
+    const Sg g = kSg[chunk - 8];
+    const uint64_t* l = lam + 264 + 65 * (chunk - 8);
+    gl::AccProd acc;
+    hphi::xor_run<false>(acc, C, g.t, [&](int b) { return C(g.bits + ((b + g.r1) & 31)); },
+                         [&](int b) { return C(g.bits + ((b + g.r2) & 31)); }, l, 0, nullptr);
+    hphi::xor_run<true>(acc, C, g.bit, [&](int b) { return C(g.t + b); },
+                        [&](int b) { return g.shift && b + g.r3 >= 32 ? 0 : C(g.bits + ((b + g.r3) & 31)); }, l + 32,
+                        g.w, l + 64);
+    *out = gl::neg(acc.reduce());
+    return;
+  }
+  if (chunk == 12) {  // Ch(e, f, g) = e f + g - e g
+    gl::AccProd acc;
+    hphi::ch_run(acc, C, BIT_E, BIT_F, BIT_G, CH_BIT, CH_W, lam + 524, lam + 556);
+    *out = gl::neg(acc.reduce());
+    return;
+  }
+  if (chunk == 13) {  // Maj(a, b, c) with auxiliaries ab, ac, bc, u = ab^ac, maj = u^bc
+    gl::AccProd acc;
+    hphi::maj_run(acc, C, BIT_A, BIT_B, BIT_C, MAJ_AB, MAJ_AC, MAJ_BC, lam + 557);
+    *out = gl::neg(acc.reduce());
+    return;
+  }
+  if (chunk == 14) {
+    gl::AccProd acc;
+    hphi::xor_run<false>(acc, C, MAJ_U, [&](int b) { return C(MAJ_AB + b); }, [&](int b) { return C(MAJ_AC + b); },
+                         lam + 653, 0, nullptr);
+    hphi::xor_run<true>(acc, C, MAJ_BIT, [&](int b) { return C(MAJ_U + b); }, [&](int b) { return C(MAJ_BC + b); },
+                        lam + 685, MAJ_W, lam + 717);
+    *out = gl::neg(acc.reduce());
+    return;
+  }
   const uint64_t j = (i + step) & (n - 1);
-  auto C = [&](uint32_t col) { return __ldg(lde + (uint64_t)col * n + i); };
-  auto X = [&](uint32_t col) { return __ldg(lde + (uint64_t)col * n + j); };
+  const hphi::Cells X{lde + j, n};
   const uint64_t row = i / row_div, blk = row / ROWS_PER_BLOCK, br = row % ROWS_PER_BLOCK;
   const bool past = blk >= n_blocks;
   const bool comp = !past && br < 64, fin = !past && br == 64, sched = !past && br >= 15 && br <= 62;
-  Acc acc{lam, 0, chunk == 0 ? 0u : chunk == 1 ? 264u : 524u};
-  // sum_b v_b 2^b over 32 columns: 96-bit terms summed exactly, one reduction
-  auto pack = [&](uint32_t off) {
-    gl::Acc128 a;
-#pragma unroll
-    for (int b = 0; b < 32; ++b) a.add_shl(C(off + b), b);
-    return a.reduce();
-  };
-  if (chunk == 0) {
-  // bit booleanity: A, B, C, E, F, G, W_win[14], W_win[1]
-  const uint32_t bool_offs[8] = {BIT_A, BIT_B, BIT_C, BIT_E, BIT_F, BIT_G, BIT_WW14, BIT_WW1};
-#pragma unroll 1
-  for (int w = 0; w < 8; ++w)
-#pragma unroll 4
-    for (int b = 0; b < 32; ++b) {
-      uint64_t v = C(bool_offs[w] + b);
-      acc.push(gl::mul(v, gl::sub(1, v)));
-    }
-  // bit -> word decompositions
-  acc.push(gl::sub(C(A_a), pack(BIT_A)));
-  acc.push(gl::sub(C(A_b), pack(BIT_B)));
-  acc.push(gl::sub(C(A_c), pack(BIT_C)));
-  acc.push(gl::sub(C(A_e), pack(BIT_E)));
-  acc.push(gl::sub(C(A_f), pack(BIT_F)));
-  acc.push(gl::sub(C(A_g), pack(BIT_G)));
-  acc.push(gl::sub(C(WW0 + 14), pack(BIT_WW14)));
-  acc.push(gl::sub(C(WW0 + 1), pack(BIT_WW1)));
-  part[i] = acc.phi;
-  return;
-  }
-  if (chunk == 1) {
-  // Sigma0(a), Sigma1(e) (rotations), sigma0(W[t-14]), sigma1(W[t-1]) (two rotations + a shift)
-  struct Sg {
-    uint32_t bits, t, bit, w;
-    int r1, r2, r3;
-    bool shift;
-  };
-  const Sg sgs[4] = {{BIT_A, S0_T, S0_BIT, S0_W, 2, 13, 22, false},
-                     {BIT_E, S1_T, S1_BIT, S1_W, 6, 11, 25, false},
-                     {BIT_WW1, SS0_T, SS0_BIT, SS0_W, 7, 18, 3, true},
-                     {BIT_WW14, SS1_T, SS1_BIT, SS1_W, 17, 19, 10, true}};
-#pragma unroll 1
-  for (int q = 0; q < 4; ++q) {
-    const Sg g = sgs[q];
-#pragma unroll 4
-    for (int b = 0; b < 32; ++b)
-      acc.push(gl::sub(C(g.t + b), xor_poly(C(g.bits + ((b + g.r1) & 31)), C(g.bits + ((b + g.r2) & 31)))));
-#pragma unroll 4
-    for (int b = 0; b < 32; ++b) {
-      uint64_t r = g.shift ? (b + g.r3 < 32 ? C(g.bits + b + g.r3) : 0) : C(g.bits + ((b + g.r3) & 31));
-      acc.push(gl::sub(C(g.bit + b), xor_poly(C(g.t + b), r)));
-    }
-    acc.push(gl::sub(C(g.w), pack(g.bit)));
-  }
-  part[n + i] = acc.phi;
-  return;
-  }
-  // Ch(e, f, g) = e f + g - e g
-#pragma unroll 4
-  for (int b = 0; b < 32; ++b) {
-    uint64_t e = C(BIT_E + b), f = C(BIT_F + b), g = C(BIT_G + b);
-    acc.push(gl::sub(C(CH_BIT + b), gl::sub(gl::add(gl::mul(e, f), g), gl::mul(e, g))));
-  }
-  acc.push(gl::sub(C(CH_W), pack(CH_BIT)));
-  // Maj(a, b, c) with auxiliaries ab, ac, bc, u = ab^ac, maj = u^bc
-#pragma unroll 4
-  for (int b = 0; b < 32; ++b) {
-    uint64_t a = C(BIT_A + b), bb = C(BIT_B + b), c = C(BIT_C + b);
-    acc.push(gl::sub(C(MAJ_AB + b), gl::mul(a, bb)));
-    acc.push(gl::sub(C(MAJ_AC + b), gl::mul(a, c)));
-    acc.push(gl::sub(C(MAJ_BC + b), gl::mul(bb, c)));
-  }
-#pragma unroll 4
-  for (int b = 0; b < 32; ++b) acc.push(gl::sub(C(MAJ_U + b), xor_poly(C(MAJ_AB + b), C(MAJ_AC + b))));
-#pragma unroll 4
-  for (int b = 0; b < 32; ++b) acc.push(gl::sub(C(MAJ_BIT + b), xor_poly(C(MAJ_U + b), C(MAJ_BC + b))));
-  acc.push(gl::sub(C(MAJ_W), pack(MAJ_BIT)));
+  hphi::Push acc{{}, lam + 718};
   // T1 = h + Sigma1 + Ch + K[t] + W[t] = T1_lo + 2^32 carry, 3 carry bits
   const uint64_t P32 = 1ull << 32;
   const uint64_t krow = comp ? kK[br] : 0;
@@ -327,14 +294,12 @@ __global__ void __launch_bounds__(128, 4) sha256_phi_kernel(const uint64_t* __re
   } else {
     acc.zeros(4);
   }
-  part[2 * n + i] = acc.phi;
+  *out = acc.acc.reduce();
 }
 
 __global__ void sha256_phi_sum(const uint64_t* __restrict__ part, uint64_t n, uint64_t* __restrict__ phi,
                                uint64_t out_stride, uint64_t out_off) {
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  phi[out_off + i * out_stride] = gl::add(gl::add(part[i], part[n + i]), part[2 * n + i]);
+  hphi::sum_parts(part, n, kPhiChunks, phi, [&](uint64_t i) { return out_off + i * out_stride; });
 }
 
 bool g_k_uploaded[64] = {false};
@@ -433,8 +398,8 @@ cudaError_t sha256_phi_points(const uint64_t* evals, uint64_t n, uint64_t step, 
   if (e != cudaSuccess) return e;
   {
     SG_LAUNCH_SCOPE("merge_phi", s);
-    sha256_phi_kernel<<<dim3((unsigned)((n + T - 1) / T), kPhiChunks), T, 0, s>>>(evals, n, step, row_div, n_blocks,
-                                                                                   lambdas, part);
+    sha256_phi_kernel<<<(unsigned)((n + T - 1) / T * kPhiChunks), T, 0, s>>>(evals, n, step, row_div, n_blocks, lambdas,
+                                                                             part);
   }
   {
     SG_LAUNCH_SCOPE("merge_phi_sum", s);

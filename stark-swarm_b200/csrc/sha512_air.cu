@@ -16,6 +16,7 @@
 
 #include "counters.hpp"
 #include "gl.cuh"
+#include "hash_phi.cuh"
 #include "sha512_air.cuh"
 
 namespace sg {
@@ -196,42 +197,40 @@ __global__ void __launch_bounds__(256) sha512_expand_kernel(const sha512::BlockW
 }
 
 // ------------------------------------------------------------------ device Phi
-struct Acc {
-  const uint64_t* lam;
-  uint64_t phi;
-  uint32_t k;
-  __device__ __forceinline__ void push(uint64_t v) {
-    phi = gl::add(phi, gl::mul(__ldg(lam + k), v));
-    ++k;
-  }
-  __device__ __forceinline__ void zeros(uint32_t cnt) { k += cnt; }  // disabled slots contribute 0
+// tables indexed by the chunk: constant memory (as local arrays they would be built on the stack)
+__constant__ uint32_t kBoolBits[8] = {sha512::BIT_A, sha512::BIT_B, sha512::BIT_C, sha512::BIT_E, sha512::BIT_F, sha512::BIT_G, sha512::BIT_WW14, sha512::BIT_WW1};
+__constant__ uint32_t kBoolWord[8] = {sha512::A_LO + 0, sha512::A_LO + 2, sha512::A_LO + 4, sha512::A_LO + 8, sha512::A_LO + 10, sha512::A_LO + 12, sha512::WW0_LO + 28, sha512::WW0_LO + 2};
+struct Sg {
+  uint32_t bits, t, bit, lo;
+  int r1, r2, r3;
+  bool shift;
 };
+__constant__ Sg kSg[4] = {{sha512::BIT_A, sha512::S0_T, sha512::S0_BIT, sha512::S0_LO, 28, 34, 39, false},
+                           {sha512::BIT_E, sha512::S1_T, sha512::S1_BIT, sha512::S1_LO, 14, 18, 41, false},
+                           {sha512::BIT_WW1, sha512::SS0_T, sha512::SS0_BIT, sha512::SS0_LO, 1, 8, 7, true},
+                           {sha512::BIT_WW14, sha512::SS1_T, sha512::SS1_BIT, sha512::SS1_LO, 19, 61, 6, true}};
 
-__device__ __forceinline__ uint64_t xor_poly(uint64_t x, uint64_t y) {
-  // x + y - 2xy
-  const uint64_t m = gl::mul(x, y);
-  return gl::sub(gl::add(x, y), gl::add(m, m));
-}
-
-// The 1526 constraints in kPhiChunks chunks (grid.y), as in the SHA-256 kernel:
-// 0-527 (bit booleanity, limb packs), 528-1047 (the four Sigma / sigma blocks),
-// 1048-1525 (the rest); chunk c writes its part of Phi at part[c n + i].
-constexpr int kPhiChunks = 3;
+// The 1526 constraints in 39 chunks of 32 to 96, one CTA each (as in the SHA-256 kernel,
+// with 64-bit words as two halves): 0-15 booleanity and limb packs of the eight words, 16-31 the
+// four Sigma / sigma blocks (first xor low and high half, second xor low and high half
+// with its limb), 32-33 Ch, 34-35 the products of Maj, 36-37 its xors, 38 the rest.
+// Chunk c writes its part of Phi at part[c count + i]. 2^17 points: 1397 -> 609 us; 2^12:
+// 149 -> 37 us (3 chunks of 128 registers left most SMs without a CTA).
+constexpr int kPhiChunks = 39;
 // Work item i < count. Without cosets (coset_len = 0) it is point i of n (a power of
 // two), cell col at lde[col * stride + i], its next row at point (i + step) mod n,
 // trace row i / row_div. With cosets it is row a = i mod rows_pc of coset c = i / rows_pc:
-// point c coset_len + a, next row c coset_len + (a + 1) mod coset_len. Chunk ch writes
-// part[ch * count + i].
-__global__ void __launch_bounds__(128, 4) sha512_phi_kernel(const uint64_t* __restrict__ lde, uint64_t n,
+// point c coset_len + a, next row c coset_len + (a + 1) mod coset_len.
+__global__ void __launch_bounds__(128, 8) sha512_phi_kernel(const uint64_t* __restrict__ lde, uint64_t n,
                                                             uint64_t stride, uint64_t count, uint64_t step,
                                                             uint64_t row_div, uint64_t n_blocks,
                                                             const uint64_t* __restrict__ lam,
                                                             uint64_t* __restrict__ part, uint64_t coset_len,
                                                             uint64_t rows_pc) {
   using namespace sha512;
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  const uint32_t chunk = blockIdx.x % kPhiChunks;
+  const uint64_t i = (blockIdx.x / kPhiChunks) * (uint64_t)blockDim.x + threadIdx.x;
   if (i >= count) return;
-  const uint32_t chunk = blockIdx.y;
   uint64_t pt, j, row;
   if (coset_len == 0) {
     pt = i;
@@ -243,92 +242,65 @@ __global__ void __launch_bounds__(128, 4) sha512_phi_kernel(const uint64_t* __re
     pt = c * coset_len + row;
     j = c * coset_len + (row + 1 == coset_len ? 0 : row + 1);
   }
-  auto C = [&](uint32_t col) { return __ldg(lde + (uint64_t)col * stride + pt); };
-  auto X = [&](uint32_t col) { return __ldg(lde + (uint64_t)col * stride + j); };
+  const hphi::Cells C{lde + pt, stride};
+  uint64_t* out = part + chunk * count + i;
+  if (chunk < 16) {
+    const uint32_t w = chunk >> 1, h = chunk & 1;
+    gl::AccProd acc;
+    hphi::bool_pack(acc, C, kBoolBits[w] + 32 * h, kBoolWord[w] + h, lam + 64 * w + 32 * h, lam + 512 + chunk);
+    *out = acc.reduce();
+    return;
+  }
+  if (chunk < 32) {
+    // Sigma0(a), Sigma1(e) (rotations), sigma0(W_win[1]), sigma1(W_win[14]) (two rotations + a shift)
+    const uint32_t q = (chunk - 16) >> 2, second = (chunk >> 1) & 1, h = chunk & 1;
+    const Sg g = kSg[q];
+    const int b0 = 32 * h;
+    const uint64_t* l = lam + 528 + 130 * q;
+    gl::AccProd acc;
+    if (!second)
+      hphi::xor_run<false>(acc, C, g.t + b0, [&](int b) { return C(g.bits + ((b0 + b + g.r1) & 63)); },
+                           [&](int b) { return C(g.bits + ((b0 + b + g.r2) & 63)); }, l + b0, 0, nullptr);
+    else
+      hphi::xor_run<true>(acc, C, g.bit + b0, [&](int b) { return C(g.t + b0 + b); },
+                          [&](int b) { return g.shift && b0 + b + g.r3 >= 64 ? 0 : C(g.bits + ((b0 + b + g.r3) & 63)); },
+                          l + 64 + b0, g.lo + h, l + 128 + h);
+    *out = gl::neg(acc.reduce());
+    return;
+  }
+  if (chunk < 34) {  // Ch(e, f, g) = e f + g - e g
+    const uint32_t b0 = 32 * (chunk & 1);
+    gl::AccProd acc;
+    hphi::ch_run(acc, C, BIT_E + b0, BIT_F + b0, BIT_G + b0, CH_BIT + b0, chunk & 1 ? CH_HI : CH_LO, lam + 1048 + b0,
+                 lam + 1112 + (chunk & 1));
+    *out = gl::neg(acc.reduce());
+    return;
+  }
+  if (chunk < 36) {  // Maj(a, b, c) with auxiliaries ab, ac, bc, u = ab^ac, maj = u^bc
+    const uint32_t b0 = 32 * (chunk & 1);
+    gl::AccProd acc;
+    hphi::maj_run(acc, C, BIT_A + b0, BIT_B + b0, BIT_C + b0, MAJ_AB + b0, MAJ_AC + b0, MAJ_BC + b0,
+                  lam + 1114 + 3 * b0);
+    *out = gl::neg(acc.reduce());
+    return;
+  }
+  if (chunk < 38) {
+    const uint32_t b0 = 32 * (chunk & 1);
+    gl::AccProd acc;
+    hphi::xor_run<false>(acc, C, MAJ_U + b0, [&](int b) { return C(MAJ_AB + b0 + b); },
+                         [&](int b) { return C(MAJ_AC + b0 + b); }, lam + 1306 + b0, 0, nullptr);
+    hphi::xor_run<true>(acc, C, MAJ_BIT + b0, [&](int b) { return C(MAJ_U + b0 + b); },
+                        [&](int b) { return C(MAJ_BC + b0 + b); }, lam + 1370 + b0, chunk & 1 ? MAJ_HI : MAJ_LO,
+                        lam + 1434 + (chunk & 1));
+    *out = gl::neg(acc.reduce());
+    return;
+  }
+  const hphi::Cells X{lde + j, stride};
   const uint64_t blk = row / ROWS_PER_BLOCK, br = row % ROWS_PER_BLOCK;
   const bool past = blk >= n_blocks;
   const bool comp = !past && br < ROUNDS, fin = !past && br == ROUNDS, sched = !past && br >= 15 && br <= 78;
-  Acc acc{lam, 0, chunk == 0 ? 0u : chunk == 1 ? 528u : 1048u};
-  // sum_{b<32} v_b 2^b over 32 columns: 96-bit terms summed exactly, one reduction
-  auto pack = [&](uint32_t off) {
-    gl::Acc128 a;
-#pragma unroll
-    for (int b = 0; b < 32; ++b) a.add_shl(C(off + b), b);
-    return a.reduce();
-  };
   const uint64_t P32 = 1ull << 32;
-  if (chunk == 0) {
-  // bit booleanity: A, B, C, E, F, G, W_win[14], W_win[1]
-  const uint32_t bool_offs[8] = {BIT_A, BIT_B, BIT_C, BIT_E, BIT_F, BIT_G, BIT_WW14, BIT_WW1};
-#pragma unroll 1
-  for (int w = 0; w < 8; ++w)
-#pragma unroll 4
-    for (int b = 0; b < 64; ++b) {
-      const uint64_t v = C(bool_offs[w] + b);
-      acc.push(gl::mul(v, gl::sub(1, v)));
-    }
-  // bit -> limb decompositions: a, b, c, e, f, g, then W_win[14], W_win[1]
-  const uint32_t limb_words[8][2] = {{A_LO + 0, BIT_A}, {A_LO + 2, BIT_B}, {A_LO + 4, BIT_C}, {A_LO + 8, BIT_E},
-                                     {A_LO + 10, BIT_F}, {A_LO + 12, BIT_G}, {WW0_LO + 28, BIT_WW14},
-                                     {WW0_LO + 2, BIT_WW1}};
-#pragma unroll 1
-  for (int q = 0; q < 8; ++q) {
-    acc.push(gl::sub(C(limb_words[q][0]), pack(limb_words[q][1])));
-    acc.push(gl::sub(C(limb_words[q][0] + 1), pack(limb_words[q][1] + 32)));
-  }
-  part[i] = acc.phi;
-  return;
-  }
-  if (chunk == 1) {
-  // Sigma0(a), Sigma1(e) (rotations), sigma0(W_win[1]), sigma1(W_win[14]) (two rotations + a shift)
-  struct Sg {
-    uint32_t bits, t, bit, lo;
-    int r1, r2, r3;
-    bool shift;
-  };
-  const Sg sgs[4] = {{BIT_A, S0_T, S0_BIT, S0_LO, 28, 34, 39, false},
-                     {BIT_E, S1_T, S1_BIT, S1_LO, 14, 18, 41, false},
-                     {BIT_WW1, SS0_T, SS0_BIT, SS0_LO, 1, 8, 7, true},
-                     {BIT_WW14, SS1_T, SS1_BIT, SS1_LO, 19, 61, 6, true}};
-#pragma unroll 1
-  for (int q = 0; q < 4; ++q) {
-    const Sg g = sgs[q];
-#pragma unroll 4
-    for (int b = 0; b < 64; ++b)
-      acc.push(gl::sub(C(g.t + b), xor_poly(C(g.bits + ((b + g.r1) & 63)), C(g.bits + ((b + g.r2) & 63)))));
-#pragma unroll 4
-    for (int b = 0; b < 64; ++b) {
-      const uint64_t r = g.shift ? (b + g.r3 < 64 ? C(g.bits + b + g.r3) : 0) : C(g.bits + ((b + g.r3) & 63));
-      acc.push(gl::sub(C(g.bit + b), xor_poly(C(g.t + b), r)));
-    }
-    acc.push(gl::sub(C(g.lo), pack(g.bit)));
-    acc.push(gl::sub(C(g.lo + 1), pack(g.bit + 32)));
-  }
-  part[count + i] = acc.phi;
-  return;
-  }
-  // Ch(e, f, g) = e f + g - e g
-#pragma unroll 4
-  for (int b = 0; b < 64; ++b) {
-    const uint64_t e = C(BIT_E + b), f = C(BIT_F + b), g = C(BIT_G + b);
-    acc.push(gl::sub(C(CH_BIT + b), gl::sub(gl::add(gl::mul(e, f), g), gl::mul(e, g))));
-  }
-  acc.push(gl::sub(C(CH_LO), pack(CH_BIT)));
-  acc.push(gl::sub(C(CH_HI), pack(CH_BIT + 32)));
-  // Maj(a, b, c) with auxiliaries ab, ac, bc, u = ab^ac, maj = u^bc
-#pragma unroll 4
-  for (int b = 0; b < 64; ++b) {
-    const uint64_t a = C(BIT_A + b), bb = C(BIT_B + b), c = C(BIT_C + b);
-    acc.push(gl::sub(C(MAJ_AB + b), gl::mul(a, bb)));
-    acc.push(gl::sub(C(MAJ_AC + b), gl::mul(a, c)));
-    acc.push(gl::sub(C(MAJ_BC + b), gl::mul(bb, c)));
-  }
-#pragma unroll 4
-  for (int b = 0; b < 64; ++b) acc.push(gl::sub(C(MAJ_U + b), xor_poly(C(MAJ_AB + b), C(MAJ_AC + b))));
-#pragma unroll 4
-  for (int b = 0; b < 64; ++b) acc.push(gl::sub(C(MAJ_BIT + b), xor_poly(C(MAJ_U + b), C(MAJ_BC + b))));
-  acc.push(gl::sub(C(MAJ_LO), pack(MAJ_BIT)));
-  acc.push(gl::sub(C(MAJ_HI), pack(MAJ_BIT + 32)));
+  hphi::Push acc{{}, lam + 1436};
   // T1 / T2 per-limb carry decompositions
   const uint64_t kt = comp ? kK512[br] : 0;
   {
@@ -424,15 +396,14 @@ __global__ void __launch_bounds__(128, 4) sha512_phi_kernel(const uint64_t* __re
   } else {
     acc.zeros(8);
   }
-  part[2 * count + i] = acc.phi;
+  *out = acc.acc.reduce();
 }
 
 __global__ void sha512_phi_sum(const uint64_t* __restrict__ part, uint64_t n, uint64_t* __restrict__ phi,
                                uint64_t out_stride, uint64_t out_off, uint64_t coset_len, uint64_t rows_pc) {
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint64_t o = coset_len ? (i / rows_pc) * coset_len + i % rows_pc : out_off + i * out_stride;
-  phi[o] = gl::add(gl::add(part[i], part[n + i]), part[2 * n + i]);
+  hphi::sum_parts(part, n, kPhiChunks, phi, [&](uint64_t i) {
+    return coset_len ? (i / rows_pc) * coset_len + i % rows_pc : out_off + i * out_stride;
+  });
 }
 
 bool g_k_uploaded[64] = {false};
@@ -533,7 +504,7 @@ cudaError_t sha512_phi_points_ex(const uint64_t* evals, uint64_t n, uint64_t str
   if (e != cudaSuccess) return e;
   {
     SG_LAUNCH_SCOPE("merge_phi", s);
-    sha512_phi_kernel<<<dim3((unsigned)((count + T - 1) / T), kPhiChunks), T, 0, s>>>(
+    sha512_phi_kernel<<<(unsigned)((count + T - 1) / T * kPhiChunks), T, 0, s>>>(
         evals, n, stride, count, step, row_div, n_blocks, lambdas, part, 0, 0);
   }
   {
@@ -558,7 +529,7 @@ cudaError_t sha512_phi_cosets(const uint64_t* evals, uint64_t n_cosets, uint64_t
   if (e != cudaSuccess) return e;
   {
     SG_LAUNCH_SCOPE("merge_phi", s);
-    sha512_phi_kernel<<<dim3((unsigned)((count + T - 1) / T), kPhiChunks), T, 0, s>>>(
+    sha512_phi_kernel<<<(unsigned)((count + T - 1) / T * kPhiChunks), T, 0, s>>>(
         evals, coset_len, n_cosets * coset_len, count, 1, 1, n_blocks, lambdas, part, coset_len, rows);
   }
   {
