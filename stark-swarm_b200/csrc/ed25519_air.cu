@@ -16,6 +16,7 @@
 #include "context.hpp"
 #include "counters.hpp"
 #include "ed25519_air.cuh"
+#include "bit_sums.cuh"
 #include "gl.cuh"
 
 namespace sg {
@@ -40,53 +41,26 @@ struct Ctx {
   const uint64_t* L;  // cell c of this point at L[c * n]
   const uint64_t* N;  // the next row's point
   uint64_t n;
-  gl::Acc128 acc;
+  gl::Acc128 acc;   // sum of lam_j C_j ..
+  gl::AccProd neg;  // .. minus this (bit columns, bit_sums.cuh)
   __device__ __forceinline__ uint64_t v(uint32_t c) const { return __ldg(L + (uint64_t)c * n); }
   __device__ __forceinline__ uint64_t w(uint32_t c) const { return __ldg(N + (uint64_t)c * n); }
   __device__ __forceinline__ void put(uint32_t lam, uint64_t x) { acc.add_mul32(lam, x); }
 };
 
-// Booleanity t_b (1 - t_b) with lambdas lam + b for the NB bit cells at bits ..,
-// added into *acc, and their pack sum_b t_b 2^b (reduced). Loads go out in
-// batches; one out-of-line copy per width keeps the instruction footprint small.
-template <int NB>
-__device__ __noinline__ uint64_t bits_pack(const uint64_t* L, uint64_t n, uint32_t bits, uint32_t lam,
-                                           gl::Acc128* acc) {
-  constexpr int H = NB > 26 ? NB / 2 : NB;
-  static_assert(NB % H == 0 && NB <= 64, "bit batch");
-  gl::Acc128 a = *acc, s;
-#pragma unroll
-  for (int h = 0; h < NB / H; ++h) {
-    uint64_t t[H];
-#pragma unroll
-    for (int j = 0; j < H; ++j) t[j] = __ldg(L + (uint64_t)(bits + h * H + j) * n);
-#pragma unroll
-    for (int j = 0; j < H; ++j) {
-      const int b = h * H + j;
-      a.add_mul32(lam + b, gl::mul(t[j], gl::sub(1, t[j])));
-      if (b < 32)
-        s.add_shl(t[j], b);
-      else
-        s.add_shl32(t[j], b - 32);
-    }
-  }
-  *acc = a;
-  return s.reduce();
-}
-
 // 255 booleanity constraints at lam + 1 .., then the 10 limb packs at lam + 256 ..
 __device__ __forceinline__ void range(Ctx& x, uint32_t limbs, uint32_t bits, uint32_t lam) {
-  gl::Acc128 a = x.acc;
+  gl::AccProd a = x.neg;
   uint32_t off = 0;
 #pragma unroll 1
   for (uint32_t i = 0; i < NL; i += 2) {
-    const uint64_t s0 = bits_pack<26>(x.L, x.n, bits + off, lam + 1 + off, &a);
-    a.add_mul32(lam + 256 + i, gl::sub(x.v(limbs + i), s0));
-    const uint64_t s1 = bits_pack<25>(x.L, x.n, bits + off + 26, lam + 1 + off + 26, &a);
-    a.add_mul32(lam + 257 + i, gl::sub(x.v(limbs + i + 1), s1));
+    bsum::range_bits<26>(x.L, x.n, bits + off, lam + 1 + off, lam + 256 + i, &a);
+    bsum::range_bits<25>(x.L, x.n, bits + off + 26, lam + 1 + off + 26, lam + 257 + i, &a);
     off += 51;
   }
-  x.acc = a;
+  x.neg = a;
+#pragma unroll
+  for (uint32_t i = 0; i < NL; ++i) x.put(lam + 256 + i, x.v(limbs + i));
 }
 
 __device__ __forceinline__ uint64_t mul_small(uint64_t x, uint32_t k) { return gl::mul(x, k); }
@@ -97,12 +71,12 @@ __device__ void eval_mul(Ctx& x, const EdBlock& g) {
   range(x, c, g.p[3], lam);
   __shared__ uint64_t s_carry[NL][kPhiThreads];
   {
-    gl::Acc128 acc = x.acc;
+    gl::AccProd neg = x.neg;
 #pragma unroll 1
     for (uint32_t k = 0; k < NL; ++k)
       s_carry[k][threadIdx.x] =
-          gl::sub(bits_pack<MUL_CB>(x.L, x.n, cy + k * MUL_CB, lam + 276 + k * MUL_CB, &acc), kMulBias);
-    x.acc = acc;
+          gl::sub(bsum::bool_pack<MUL_CB>(x.L, x.n, cy + k * MUL_CB, lam + 276 + k * MUL_CB, &neg), kMulBias);
+    x.neg = neg;
   }
   uint64_t al[NL], bl[NL];
 #pragma unroll
@@ -110,24 +84,28 @@ __device__ void eval_mul(Ctx& x, const EdBlock& g) {
     al[i] = x.v(a + i);
     bl[i] = x.v(b + i);
   }
-  // diagonals: lo[k] = sum_{i+j=k} f a_i b_j, hi[k] = sum_{i+j=k+10} f a_i b_j, f = 2 for odd i, j
-  uint64_t lo[NL], hi[NL];
+  // limb k: sum over i + j = k of f a_i b_j plus 19 times that over i + j = k + 10, f = 2 for
+  // odd i and j; ten unreduced products and one reduction
+  uint64_t b19[NL];
 #pragma unroll
-  for (uint32_t k = 0; k < NL; ++k) lo[k] = hi[k] = 0;
-#pragma unroll
-  for (uint32_t i = 0; i < NL; ++i)
-#pragma unroll
-    for (uint32_t j = 0; j < NL; ++j) {
-      uint64_t p = gl::mul(al[i], bl[j]);
-      if ((i & 1) && (j & 1)) p = gl::add(p, p);
-      if (i + j < NL)
-        lo[i + j] = gl::add(lo[i + j], p);
-      else
-        hi[i + j - NL] = gl::add(hi[i + j - NL], p);
-    }
+  for (uint32_t i = 0; i < NL; ++i) b19[i] = mul_small(bl[i], 19);
 #pragma unroll
   for (uint32_t k = 0; k < NL; ++k) {
-    const uint64_t t = gl::add(lo[k], mul_small(hi[k], 19));
+    gl::AccProd sum, odd;
+#pragma unroll
+    for (uint32_t i = 0; i < NL; ++i) {
+      const uint32_t j = (k + NL - i) % NL;
+      const uint64_t bj = i > k ? b19[j] : bl[j];
+      if ((i & 1) && (j & 1))
+        odd.add(al[i], bj);
+      else
+        sum.add(al[i], bj);
+    }
+    uint64_t t = sum.reduce();
+    if (!(k & 1)) {  // odd i and j only meet at an even k
+      const uint64_t o = odd.reduce();
+      t = gl::add(gl::add(t, o), o);
+    }
     const uint64_t cin = k == 0 ? mul_small(s_carry[NL - 1][threadIdx.x], 19) : s_carry[k - 1][threadIdx.x];
     const uint64_t v = gl::sub(gl::add(t, cin), gl::add(x.v(c + k), gl::mul_pow2(s_carry[k][threadIdx.x], (k & 1) ? 25u : 26u)));
     x.put(lam + 266 + k, v);
@@ -245,19 +223,19 @@ __device__ void eval_reduce(Ctx& x, const EdBlock& g) {
                  cnt[3] = {RED_Q, RED_R, RED_R}, base[3] = {0, 289, 561};
   for (int part = 0; part < 3; ++part)
     for (uint32_t i = 0; i < cnt[part]; ++i) {
-      gl::Acc128 a = x.acc;
-      const uint64_t s = bits_pack<RED_LB>(x.L, x.n, bits[part] + i * RED_LB, lam + 1 + base[part] + i * RED_LB, &a);
-      x.acc = a;
+      gl::AccProd a = x.neg;
+      const uint64_t s = bsum::bool_pack<RED_LB>(x.L, x.n, bits[part] + i * RED_LB, lam + 1 + base[part] + i * RED_LB, &a);
+      x.neg = a;
       x.put(lam + 1 + base[part] + cnt[part] * RED_LB + i, gl::sub(x.v(limbs[part] + i), s));
     }
   constexpr uint32_t L16[RED_R] = {0xd3ed, 0x5cf5, 0x631a, 0x5812, 0x9cd6, 0xa2f7, 0xf9de, 0x14de,
                                    0,      0,      0,      0,      0,      0,      0,      0x1000};
   uint64_t prev = 0;
   for (uint32_t k = 0; k < RED_PROD; ++k) {
-    gl::Acc128 a = x.acc;
-    const uint64_t cy = gl::sub(bits_pack<RED_CB>(x.L, x.n, g.p[7] + k * RED_CB, lam + 1 + 882 + k * RED_CB, &a),
+    gl::AccProd a = x.neg;
+    const uint64_t cy = gl::sub(bsum::bool_pack<RED_CB>(x.L, x.n, g.p[7] + k * RED_CB, lam + 1 + 882 + k * RED_CB, &a),
                                 kRedBias);
-    x.acc = a;
+    x.neg = a;
     uint64_t ql = 0;
     for (uint32_t i = 0; i < RED_Q; ++i)
       if (k >= i && k - i < RED_R && L16[k - i]) ql = gl::add(ql, gl::mul(x.v(g.p[1] + i), L16[k - i]));
@@ -272,10 +250,10 @@ __device__ void eval_reduce(Ctx& x, const EdBlock& g) {
 __device__ void eval_format(Ctx& x, const EdBlock& g) {
   const uint32_t db = g.p[0], in = g.p[1], h0 = g.p[2], lam = g.lam;
   for (uint32_t k = 0; k < 8; ++k) {
-    gl::Acc128 a = x.acc;
-    const uint64_t lo = bits_pack<32>(x.L, x.n, db + 64 * k, lam + 1 + 64 * k, &a);
-    const uint64_t hi = bits_pack<32>(x.L, x.n, db + 64 * k + 32, lam + 1 + 64 * k + 32, &a);
-    x.acc = a;
+    gl::AccProd a = x.neg;
+    const uint64_t lo = bsum::bool_pack<32>(x.L, x.n, db + 64 * k, lam + 1 + 64 * k, &a);
+    const uint64_t hi = bsum::bool_pack<32>(x.L, x.n, db + 64 * k + 32, lam + 1 + 64 * k + 32, &a);
+    x.neg = a;
     x.put(lam + 1 + 512 + 2 * k, gl::sub(x.v(h0 + 2 * k), lo));
     x.put(lam + 1 + 512 + 2 * k + 1, gl::sub(x.v(h0 + 2 * k + 1), hi));
   }
@@ -291,6 +269,7 @@ __device__ void eval_format(Ctx& x, const EdBlock& g) {
     }
 }
 
+// 128 registers: 0.71 ms for n0 = 32768 (1.04 before the unreduced sums), 0.75 at 96
 __global__ void __launch_bounds__(kPhiThreads, 4) ed25519_phi_kernel(EdPhi a, uint64_t* part) {
   const uint64_t i = blockIdx.x * (uint64_t)kPhiThreads + threadIdx.x;
   if (i >= a.n) return;
@@ -306,7 +285,7 @@ __global__ void __launch_bounds__(kPhiThreads, 4) ed25519_phi_kernel(EdPhi a, ui
   const uint32_t cls = a.row_class[row], c0 = a.cls_chunk[cls], nch = a.cls_chunk[cls + 1] - c0;
   const uint32_t ch = blockIdx.y;
   if (ch >= nch) return;
-  Ctx x{a.lde + i, a.lde + nx, a.n, {}};
+  Ctx x{a.lde + i, a.lde + nx, a.n, {}, {}};
   const uint32_t b0 = a.chunk_rng[2 * (c0 + ch)], b1 = a.chunk_rng[2 * (c0 + ch) + 1];
   for (uint32_t bi = b0; bi < b1; ++bi) {
     const EdBlock g = a.blocks[a.cls_list[bi]];
@@ -328,7 +307,7 @@ __global__ void __launch_bounds__(kPhiThreads, 4) ed25519_phi_kernel(EdPhi a, ui
       default: break;
     }
   }
-  part[(uint64_t)ch * a.n + i] = x.acc.reduce();
+  part[(uint64_t)ch * a.n + i] = gl::sub(x.acc.reduce(), x.neg.reduce());
 }
 
 __global__ void ed25519_phi_sum(EdPhi a, const uint64_t* part, uint64_t* phi) {

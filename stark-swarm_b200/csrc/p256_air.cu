@@ -15,6 +15,7 @@
 
 #include "context.hpp"
 #include "counters.hpp"
+#include "bit_sums.cuh"
 #include "gl.cuh"
 #include "p256_air.cuh"
 #include "p256_cells.cuh"
@@ -40,54 +41,32 @@ __global__ void p256_expand_kernel(P256Dev d, uint64_t k, uint64_t* trace) {
 struct Ctx {
   const uint64_t* L;  // column 0 at this point: cell c is L[c * n]
   uint64_t n;
-  gl::Acc128 acc;
+  gl::Acc128 acc;   // sum of lam_j C_j ..
+  gl::AccProd neg;  // .. minus this (bit columns, bit_sums.cuh)
   __device__ __forceinline__ uint64_t v(uint32_t c) const { return __ldg(L + (uint64_t)c * n); }
   __device__ __forceinline__ void put(uint64_t lam, uint64_t c) { acc.add_mul32((uint32_t)lam, c); }
 };
 
-// 128 threads and at most 128 registers: 4 CTAs (16 warps) per SM. Measured for
-// n = 8192: 3.8 ms, against 4.0 ms at 3 CTAs (168 registers) and 4.1 ms at 5 (96).
+// 128 threads and at most 96 registers: 5 CTAs (20 warps) per SM. Measured for
+// n = 8192: 2.98 ms, against 3.36 ms at 4 CTAs (128 registers) and 3.16 ms at 6 (80);
+// 4.75 ms before the unreduced sums (bit_sums.cuh, and the slot identities' products).
 constexpr int kPhiThreads = 128;
-
-// Booleanity terms t_b (1 - t_b) with lambdas lam + b for the NB bit cells
-// bits .. bits+NB-1, added into *acc, and the pack sum_b t_b 2^b (reduced). The
-// loads of a batch go out together. One out-of-line copy serves every range
-// check and carry: inlined at each, the unrolled bodies overflowed the
-// instruction cache.
-template <int NB>
-__device__ __noinline__ uint64_t bits_pack(const uint64_t* L, uint64_t n, uint32_t bits, uint32_t lam,
-                                           gl::Acc128* acc) {
-  constexpr int H = NB > LB ? NB / 2 : NB;  // loads per batch: 26, or 2 x 18 for a 36-bit carry
-  static_assert(NB % H == 0 && NB <= 64, "bit batch");
-  gl::Acc128 a = *acc, s;
-#pragma unroll
-  for (int h = 0; h < NB / H; ++h) {
-    uint64_t t[H];
-#pragma unroll
-    for (int j = 0; j < H; ++j) t[j] = __ldg(L + (uint64_t)(bits + h * H + j) * n);
-#pragma unroll
-    for (int j = 0; j < H; ++j) {
-      const int b = h * H + j;
-      a.add_mul32(lam + b, gl::mul(t[j], gl::sub(1, t[j])));
-      if (b < 32)
-        s.add_shl(t[j], b);
-      else
-        s.add_shl32(t[j], b - 32);
-    }
-  }
-  *acc = a;
-  return s.reduce();
-}
 
 // booleanity of the 260 bits at lam .. lam+259, limb packs at lam+260 .. lam+269
 __device__ __forceinline__ void range(Ctx& x, uint32_t limbs, uint32_t bits, uint64_t lam) {
-  gl::Acc128 a = x.acc;
+  gl::AccProd a = x.neg;
 #pragma unroll 1
-  for (uint32_t i = 0; i < NL; ++i) {
-    const uint64_t s = bits_pack<LB>(x.L, x.n, bits + i * LB, (uint32_t)(lam + i * LB), &a);
-    a.add_mul32((uint32_t)(lam + NL * LB + i), gl::sub(x.v(limbs + i), s));
-  }
-  x.acc = a;
+  for (uint32_t i = 0; i < NL; ++i)
+    bsum::range_bits<LB>(x.L, x.n, bits + i * LB, (uint32_t)(lam + i * LB), (uint32_t)(lam + NL * LB + i), &a);
+  x.neg = a;
+#pragma unroll
+  for (uint32_t i = 0; i < NL; ++i) x.put(lam + NL * LB + i, x.v(limbs + i));
+}
+
+// limb i of p, known at compile time in unrolled loops
+__device__ constexpr uint32_t p_limb(uint32_t i) {
+  constexpr uint32_t t[NL] = {0x3FFFFFF, 0x3FFFFFF, 0x3FFFFFF, 0x003FFFF, 0, 0, 0, 0x0000400, 0x3FF0000, 0x03FFFFF};
+  return t[i];
 }
 
 __device__ void eval_mul(Ctx& x, const Gadget& g, uint64_t lam) {
@@ -99,13 +78,13 @@ __device__ void eval_mul(Ctx& x, const Gadget& g, uint64_t lam) {
   __shared__ uint64_t s_carry[MUL_CP][kPhiThreads];
   const uint64_t lam_b = lam + 2 * ELEM + MUL_SP;
   {
-    gl::Acc128 acc = x.acc;
+    gl::AccProd neg = x.neg;
 #pragma unroll 1
     for (uint32_t k = 0; k < MUL_CP; ++k)
       s_carry[k][threadIdx.x] =
-          gl::sub(bits_pack<MUL_CB>(x.L, x.n, cy + k * MUL_CB, (uint32_t)(lam_b + k * MUL_CB), &acc),
+          gl::sub(bsum::bool_pack<MUL_CB>(x.L, x.n, cy + k * MUL_CB, (uint32_t)(lam_b + k * MUL_CB), &neg),
                   1ull << (MUL_CB - 1));
-    x.acc = acc;
+    x.neg = neg;
   }
   uint64_t al[NL], bl[NL], ql[NL];
 #pragma unroll
@@ -116,14 +95,16 @@ __device__ void eval_mul(Ctx& x, const Gadget& g, uint64_t lam) {
   }
 #pragma unroll
   for (uint32_t k = 0; k < MUL_SP; ++k) {
-    uint64_t ab = 0, qp = 0;
+    // sum a_i b_(k-i) and sum q_i p_(k-i) unreduced (p's limbs are below 2^26, three of them zero)
+    gl::AccProd ab;
+    gl::Acc128 qp;
 #pragma unroll
     for (uint32_t i = 0; i < NL; ++i) {
       if (i + NL - 1 < k || i > k) continue;
-      ab = gl::add(ab, gl::mul(al[i], bl[k - i]));
-      qp = gl::add(qp, gl::mul(ql[i], kPT[k - i]));
+      ab.add(al[i], bl[k - i]);
+      if (p_limb(k - i)) qp.add_mul32(p_limb(k - i), ql[i]);
     }
-    uint64_t v = gl::sub(ab, qp);
+    uint64_t v = gl::sub(ab.reduce(), qp.reduce());
     if (k < NL) v = gl::sub(v, x.v(c + k));
     if (k > 0) v = gl::add(v, s_carry[k - 1][threadIdx.x]);
     if (k < MUL_CP) v = gl::sub(v, gl::mul_pow2(s_carry[k][threadIdx.x], LB));
@@ -235,11 +216,11 @@ __device__ void eval_tail(Ctx& x, const uint64_t* nxt, const uint32_t* tail, boo
   }
 }
 
-__global__ void __launch_bounds__(kPhiThreads, 4) p256_phi_kernel(P256Phi a, uint64_t* part) {
+__global__ void __launch_bounds__(kPhiThreads, 5) p256_phi_kernel(P256Phi a, uint64_t* part) {
   const uint64_t i = blockIdx.x * (uint64_t)kPhiThreads + threadIdx.x;
   if (i >= a.n) return;
   const uint32_t ch = blockIdx.y;
-  Ctx x{a.lde + i, a.n, {}};
+  Ctx x{a.lde + i, a.n, {}, {}};
   const uint32_t g0 = a.chunk[ch], g1 = a.chunk[ch + 1];
   for (uint32_t gi = g0; gi < g1; ++gi) {
     const Gadget g = a.table[gi];
@@ -264,7 +245,7 @@ __global__ void __launch_bounds__(kPhiThreads, 4) p256_phi_kernel(P256Phi a, uin
     }
     eval_tail(x, a.lde + nx, a.tail, row + 1 == a.n_trace, row + 1 < a.n_trace, (uint64_t)a.lam_tail + 1);
   }
-  part[(uint64_t)ch * a.n + i] = x.acc.reduce();
+  part[(uint64_t)ch * a.n + i] = gl::sub(x.acc.reduce(), x.neg.reduce());
 }
 
 __global__ void p256_sum_kernel(const uint64_t* part, uint64_t n, uint32_t chunks, uint64_t* phi, uint64_t coset_len,
