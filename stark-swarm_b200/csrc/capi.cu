@@ -229,6 +229,13 @@ void sg_ctx_destroy(sg_ctx* c) {
     cudaStreamSynchronize(c->stir_stream);
     cudaStreamDestroy(c->stir_stream);
   }
+  for (cudaStream_t x : c->side)
+    if (x) {
+      cudaStreamSynchronize(x);
+      cudaStreamDestroy(x);
+    }
+  for (cudaEvent_t x : c->side_ev)
+    if (x) cudaEventDestroy(x);
   if (c->stir_in) cudaEventDestroy(c->stir_in);
   if (c->stir_out) cudaEventDestroy(c->stir_out);
   sg::pinned_release(c);

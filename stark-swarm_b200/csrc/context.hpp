@@ -28,6 +28,10 @@ struct sg_ctx {
   // phase of a proof and the two events that order it after and before `stream`.
   cudaStream_t stir_stream = nullptr;
   cudaEvent_t stir_in = nullptr, stir_out = nullptr;
+  // STIR: streams beside the one a proof runs on, for a layer's tree and for its transform and
+  // out-of-domain sums, and their events (made on first use, with that stream's priority)
+  cudaStream_t side[2] = {nullptr, nullptr};
+  cudaEvent_t side_ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   // grow-only pinned host staging for witnesses copied to the device (pinned_host)
   void* pinned = nullptr;
   size_t pinned_bytes = 0;

@@ -527,6 +527,48 @@ std::vector<uint8_t> classic_prove_device(sg_ctx* c, const uint64_t* d_f0, uint6
 
 namespace {
 
+// A proof's stream s and the context's two side streams. Work on a side stream starts
+// after what `fork` saw on s; the destructor lets s wait for both, so that buffers (freed
+// in s's order) outlive what uses them, on every way out.
+struct SideStreams {
+  sg_ctx* c;
+  cudaStream_t s, tree, ood;
+  explicit SideStreams(sg_ctx* ctx) : c(ctx), s(ctx->stream) {
+    int prio = 0;
+    cuda_check(cudaStreamGetPriority(s, &prio), "stream priority");
+    for (auto& x : c->side)
+      if (!x) cuda_check(cudaStreamCreateWithPriority(&x, cudaStreamNonBlocking, prio), "side stream");
+    for (auto& e : c->side_ev)
+      if (!e) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+    tree = c->side[0];
+    ood = c->side[1];
+  }
+  void fork() {
+    cuda_check(cudaEventRecord(c->side_ev[0], s), "event");
+    cuda_check(cudaStreamWaitEvent(tree, c->side_ev[0], 0), "wait");
+    cuda_check(cudaStreamWaitEvent(ood, c->side_ev[0], 0), "wait");
+  }
+  // a layer's results are on their way to the host; `collect` waits for them
+  void results(uint64_t ell) {
+    cuda_check(cudaEventRecord(c->side_ev[2 + (ell & 1)], tree), "event");
+    cuda_check(cudaEventRecord(c->side_ev[4 + (ell & 1)], ood), "event");
+  }
+  void collect(uint64_t ell) {
+    cuda_check(cudaEventSynchronize(c->side_ev[2 + (ell & 1)]), "sync");
+    cuda_check(cudaEventSynchronize(c->side_ev[4 + (ell & 1)]), "sync");
+  }
+  ~SideStreams() {
+    for (cudaStream_t x : {tree, ood})
+      if (cudaEventRecord(c->side_ev[1], x) == cudaSuccess) cudaStreamWaitEvent(s, c->side_ev[1], 0);
+  }
+};
+
+// Per layer the transcript needs the layer's root and its out-of-domain values; the fold
+// needs the challenge that follows from the layer before. So the three run on streams of
+// their own: folds on s, tree levels on the second, transform and out-of-domain sums on
+// the third, and the host takes layer l - 1's results while layer l's are in the making.
+// (These kernels are short and latency-bound, and ran one after another with the host
+// waiting in between.)
 std::vector<uint8_t> stir_prove_on_stream(sg_ctx* c, const uint64_t* d_f0, uint64_t n0, const sg_fri_params& p) {
   cudaStream_t s = c->stream;
   const uint64_t L = p.schedule_len;
@@ -549,19 +591,6 @@ std::vector<uint8_t> stir_prove_on_stream(sg_ctx* c, const uint64_t* d_f0, uint6
   HostTranscript tr("FRI/FS");
   bind_statement(tr, p, n0);
 
-  // packed f0 tree: leaf b = {f0[b + j n0/m0]}_j (fri.rs:1420-1431), label 0xFF
-  const uint64_t m0 = p.schedule[0], nn0 = n0 / m0;
-  Tree f0t;
-  f0t.make(nn0, layer_arities(nn0, 16), 0xFF, s);
-  cuda_check(tree_hash_leaves(f0t.t, d_f0, (uint32_t)m0, nn0, 0, s), "f0 leaves");
-  cuda_check(tree_hash_levels(f0t.t, s), "f0 levels");
-  std::vector<uint64_t> h;
-  d2h(&h, f0t.t.d + DL * f0t.t.off.back(), DL, s);
-  cuda_check(cudaStreamSynchronize(s), "sync");
-  pr.root_f0 = digest_at(h, 0);
-  tr.absorb_bytes(pr.root_f0.data(), HB);
-  const gl::Fp6 z = tr.challenge_ext("z_fp3");
-
   const uint64_t work = std::max<uint64_t>(n0, 6 * sizes[1]);
   uint64_t scratch_len = ntt_scratch_elems(1, log2_exact(n0));
   for (uint64_t i = 1; i <= L; ++i) scratch_len = std::max(scratch_len, ntt_scratch_elems(6, log2_exact(sizes[i])));
@@ -573,30 +602,76 @@ std::vector<uint8_t> stir_prove_on_stream(sg_ctx* c, const uint64_t* d_f0, uint6
   std::vector<DBuf> planes(L + 1);
   std::vector<Tree> trees(L);
   DBuf tuples;
-  Tree ctree;
+  Tree f0t, ctree;
+  // per layer, in pinned host memory: the m evaluations, then the root
+  constexpr uint64_t kRes = 16 * 6 + DL;
+  uint64_t* res = (uint64_t*)pinned_host(c, (L * kRes + DL) * 8);
+  SideStreams side(c);  // (declared after the buffers: joined before they are freed)
 
+  // The tree over the 6 components of f_l (label l; for l >= 1 the fold before has written
+  // its leaves) on one side stream, the coefficients and out-of-domain values on the other.
   const uint64_t* cur = d_f0;
   bool base = true;
+  auto start_tree = [&](uint64_t ell) {
+    cuda_check(tree_hash_levels(trees[ell].t, side.tree), "layer levels");
+    cuda_check(cudaMemcpyAsync(res + ell * kRes + 16 * 6, trees[ell].t.d + DL * trees[ell].t.off.back(), DL * 8,
+                               cudaMemcpyDeviceToHost, side.tree),
+               "d2h");
+  };
+  auto start_coef = [&](uint64_t ell) {
+    const uint64_t n = sizes[ell];
+    cuda_check(ntt_batch(c->tw, cur, coef.p, base ? 1 : 6, n, n, (int)log2_exact(n), true, n, scratch.p, side.ood),
+               "ntt");
+  };
+  auto start_ood = [&](uint64_t ell, const gl::Fp6& zc) {
+    const uint64_t n = sizes[ell], m = p.schedule[ell];
+    cuda_check(ood_evaluate(coef.p, base, n, (int)m, zc, partials.p, evals.p, side.ood), "ood");
+    cuda_check(cudaMemcpyAsync(res + ell * kRes, evals.p, m * 6 * 8, cudaMemcpyDeviceToHost, side.ood), "d2h");
+    side.results(ell);
+  };
+  // the layer's evaluations and root into the proof and the transcript
+  auto take_layer = [&](uint64_t ell) {
+    side.collect(ell);
+    const uint64_t m = p.schedule[ell];
+    const uint64_t* ev = res + ell * kRes;
+    std::vector<gl::Fp6> evs(m);
+    for (uint64_t j = 0; j < m; ++j)
+      for (int q = 0; q < 6; ++q) evs[j].c[q] = ev[j * 6 + q];
+    pr.fz.push_back(evs[0]);
+    for (auto& e : evs) tr.absorb_ext(e);
+    pr.coset_evals.push_back(std::move(evs));
+    Digest root;
+    memcpy(root.data(), ev + 16 * 6, HB);
+    pr.roots.push_back(root);
+    tr.absorb_bytes(root.data(), HB);
+  };
+
+  // packed f0 tree: leaf b = {f0[b + j n0/m0]}_j (fri.rs:1420-1431), label 0xFF; beside it
+  // layer 0's tree and transform, which wait for no challenge
+  const uint64_t m0 = p.schedule[0], nn0 = n0 / m0;
+  f0t.make(nn0, layer_arities(nn0, 16), 0xFF, s);
+  trees[0].make(n0, layer_arities(n0, m0), 0, s);
+  side.fork();
+  cuda_check(tree_hash_leaves(f0t.t, d_f0, (uint32_t)m0, nn0, 0, s), "f0 leaves");
+  cuda_check(tree_hash_levels(f0t.t, s), "f0 levels");
+  cuda_check(cudaMemcpyAsync(res + L * kRes, f0t.t.d + DL * f0t.t.off.back(), DL * 8, cudaMemcpyDeviceToHost, s), "d2h");
+  cuda_check(tree_hash_leaves(trees[0].t, d_f0, 1, n0, 5, side.tree), "layer-0 leaves");
+  start_tree(0);
+  start_coef(0);
+  cuda_check(cudaStreamSynchronize(s), "sync");
+  memcpy(pr.root_f0.data(), res + L * kRes, HB);
+  tr.absorb_bytes(pr.root_f0.data(), HB);
+  const gl::Fp6 z = tr.challenge_ext("z_fp3");
+
   gl::Fp6 zc = z;
   for (uint64_t ell = 0; ell < L; ++ell) {
     const uint64_t m = p.schedule[ell], n = sizes[ell], nn = n / m;
     const unsigned lg = log2_exact(n);
     const bool last_cc = use_cc && ell == L - 1;
+    start_ood(ell, zc);
+    if (ell > 0) take_layer(ell - 1);
     gl::Fp6 alpha = gl::e_zero();
     if (!last_cc) alpha = tr.challenge_ext("alpha");
-
-    // layer tree (label ell) over the 6 components of f_ell; for ell >= 1 the
-    // previous fold already wrote its leaves
-    if (ell == 0) {
-      trees[0].make(n, layer_arities(n, m), 0, s);
-      cuda_check(tree_hash_leaves(trees[0].t, d_f0, 1, n, 5, s), "layer-0 leaves");
-    }
-    cuda_check(tree_hash_levels(trees[ell].t, s), "layer levels");
-
-    // out-of-domain coset evaluation
-    const uint32_t cols = base ? 1 : 6;
-    ntt(c, cur, coef.p, cols, n, n, lg, true, n, scratch.p);
-    cuda_check(ood_evaluate(coef.p, base, n, (int)m, zc, partials.p, evals.p, s), "ood");
 
     FoldArgs fa{};
     fa.f = cur;
@@ -607,8 +682,8 @@ std::vector<uint8_t> stir_prove_on_stream(sg_ctx* c, const uint64_t* d_f0, uint6
     fa.alpha = alpha;
     fa.tw_inv_lo = c->tw.d_inv_lo;
     fa.tw_inv_hi = c->tw.d_inv_hi;
+    planes[ell + 1].alloc(6 * nn, s);
     if (!last_cc) {
-      planes[ell + 1].alloc(6 * nn, s);
       fa.next = planes[ell + 1].p;
       if (ell + 1 < L) {
         trees[ell + 1].make(nn, layer_arities(nn, p.schedule[ell + 1]), ell + 1, s);
@@ -624,26 +699,11 @@ std::vector<uint8_t> stir_prove_on_stream(sg_ctx* c, const uint64_t* d_f0, uint6
       ctree.make(nn, layer_arities(nn, 16), 0xFE, s);
       cuda_check(tree_hash_leaves(ctree.t, tuples.p, (uint32_t)(6 * m), nn, 0, s), "coeff leaves");
       cuda_check(tree_hash_levels(ctree.t, s), "coeff levels");
-    }
-
-    std::vector<uint64_t> ev, root, croot, tup;
-    d2h(&ev, evals.p, m * 6, s);
-    d2h(&root, trees[ell].t.d + DL * trees[ell].t.off.back(), DL, s);
-    if (last_cc) {
+      std::vector<uint64_t> croot, tup;
       d2h(&croot, ctree.t.d + DL * ctree.t.off.back(), DL, s);
       d2h(&tup, tuples.p, 6 * m * nn, s);
-    }
-    cuda_check(cudaStreamSynchronize(s), "sync");
-    std::vector<gl::Fp6> evs(m);
-    for (uint64_t j = 0; j < m; ++j)
-      for (int q = 0; q < 6; ++q) evs[j].c[q] = ev[j * 6 + q];
-    pr.fz.push_back(evs[0]);
-    for (auto& e : evs) tr.absorb_ext(e);
-    pr.coset_evals.push_back(std::move(evs));
-    pr.roots.push_back(digest_at(root, 0));
-    tr.absorb_bytes(pr.roots.back().data(), HB);
-    zc = gl::e_pow(zc, m);
-    if (last_cc) {
+      take_layer(ell);
+      cuda_check(cudaStreamSynchronize(s), "sync");
       pr.has_ct = pr.has_croot = true;
       pr.coeff_root = digest_at(croot, 0);
       tr.absorb_bytes(pr.coeff_root.data(), HB);
@@ -653,13 +713,21 @@ std::vector<uint8_t> stir_prove_on_stream(sg_ctx* c, const uint64_t* d_f0, uint6
       for (uint64_t b = 0; b < nn; ++b)
         for (uint64_t k = 0; k < m; ++k)
           for (int q = 0; q < 6; ++q) pr.coeff_tuples[b][k].c[q] = tup[(k * 6 + q) * nn + b];
-      planes[ell + 1].alloc(6 * nn, s);
       cuda_check(fold_tuples(tuples.p, nn, (int)m, alpha, planes[ell + 1].p, s), "final fold");
     }
     cur = planes[ell + 1].p;
     base = false;
+    zc = gl::e_pow(zc, m);
+    if (ell + 1 < L) {
+      side.fork();
+      start_tree(ell + 1);
+      start_coef(ell + 1);
+    } else if (!last_cc) {
+      take_layer(ell);
+    }
   }
 
+  // (every layer's results have been collected, so coef is free)
   // final polynomial coefficients (fri.rs:1915-1935)
   const uint64_t nf = sizes[L];
   const unsigned lgf = log2_exact(nf);
