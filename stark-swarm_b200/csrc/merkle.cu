@@ -145,11 +145,14 @@ __global__ void node_kernel(const uint64_t* child, uint64_t n_child, uint64_t* p
 
 // Keccak-f[1600] by one warp: thread t < 25 holds state lane A[t] (t = x + 5y) and
 // the others follow along with lanes they never hand out. Per round, theta's column
-// parities and D, pi's lane move and chi's two neighbours are warp shuffles, rho is
-// the thread's own rotation. About 33 instructions a round for the warp against
-// some 260 for one thread holding the whole state, so a lone permutation (the
-// narrow top levels of a tree) finishes about three times sooner. The rotation
-// offsets and round constants are Keccak's (FIPS 202, section 3.2).
+// parities and D are two rounds of warp shuffles, rho is the thread's own rotation, and
+// chi's three lanes come in a third round from where they stand before pi. Bound by the
+// latency of these three exchanges (26 clk for a shuffle and 3 for each further one):
+// 190 clk a round, against 430 to 470 for one thread holding the whole state (ALU rate).
+// Four rounds unrolled: 221 clk with one, 202 with two, 183 with twelve, for three times the
+// code; all ten lanes of both neighbour columns in one exchange, or the exchange through
+// shared memory: 15 to 20 % slower. The rotation offsets and round constants are Keccak's
+// (FIPS 202, section 3.2).
 __constant__ uint8_t kRhoOff[25] = {0, 1, 62, 28, 27, 36, 44, 6, 55, 20, 3, 10, 43, 25, 39,
                                     41, 45, 15, 21, 8, 18, 2, 61, 56, 14};
 
@@ -159,24 +162,31 @@ __device__ __forceinline__ uint64_t shfl64(uint64_t v, int src) {
   return (uint64_t)hi << 32 | lo;
 }
 
-__device__ __forceinline__ uint64_t rotl_var(uint64_t v, uint32_t n) { return n ? (v << n) | (v >> (64 - n)) : v; }
+// rotation by n = 32 swap + r, r < 32: a funnel shift by 0 leaves its word as it is
+__device__ __forceinline__ uint64_t rotl_var(uint64_t v, bool swap, uint32_t r) {
+  const uint32_t a = (uint32_t)v, b = (uint32_t)(v >> 32), lo = swap ? b : a, hi = swap ? a : b;
+  return (uint64_t)__funnelshift_l(lo, hi, r) << 32 | __funnelshift_l(hi, lo, r);
+}
 
 __device__ void keccak_f_warp(uint64_t& a, int t) {
   const int x = t % 5, y = (t / 5) % 5;
   const int s1 = x + 5 * ((y + 1) % 5), s2 = x + 5 * ((y + 2) % 5), s3 = x + 5 * ((y + 3) % 5),
             s4 = x + 5 * ((y + 4) % 5);
   const int cm = (x + 4) % 5, cp = (x + 1) % 5;
-  // pi: the lane landing at (x, y) comes from (x', y') = (3 (y - 3x) mod 5, x)
-  const int pi = (3 * (y - 3 * x) % 5 + 5) % 5 + 5 * x;
-  const int n1 = (x + 1) % 5 + 5 * y, n2 = (x + 2) % 5 + 5 * y;
-  const uint32_t rho = t < 25 ? kRhoOff[t] : 0;
-#pragma unroll 1
+  // pi: the lane landing at (x, y) comes from (x', y') = (3 (y - 3x) mod 5, x). Chi at
+  // (x, y) takes the lanes that land at x, x + 1 and x + 2 of its row: each is fetched
+  // from where it stands before pi.
+  const auto from = [y](int X) { return (3 * (y - 3 * X) % 5 + 5) % 5 + 5 * X; };
+  const int p0 = from(x), p1 = from((x + 1) % 5), p2 = from((x + 2) % 5);
+  const uint32_t rho = t < 25 ? kRhoOff[t] : 0, rr = rho & 31;
+  const bool swap = rho >= 32;
+  const uint64_t iota = t == 0 ? ~0ull : 0;
+#pragma unroll 4
   for (int r = 0; r < 24; ++r) {
     const uint64_t c = kc::xor3(kc::xor3(a, shfl64(a, s1), shfl64(a, s2)), shfl64(a, s3), shfl64(a, s4));
     a = kc::xor3(a, shfl64(c, cm), kc::rotl(shfl64(c, cp), 1));
-    const uint64_t b = shfl64(rotl_var(a, rho), pi);
-    a = kc::chi(b, shfl64(b, n1), shfl64(b, n2));
-    if (t == 0) a ^= kc::kRC_dev[r];
+    const uint64_t b = rotl_var(a, swap, rr);
+    a = kc::chi(shfl64(b, p0), shfl64(b, p1), shfl64(b, p2)) ^ (kc::kRC_dev[r] & iota);
   }
 }
 
@@ -186,43 +196,44 @@ __device__ void keccak_f_warp(uint64_t& a, int t) {
 __device__ void node_hash_warp(const uint64_t* child, uint64_t n_child, uint64_t* parent, uint64_t p,
                                uint32_t arity, uint64_t level, uint64_t label, int t) {
   const uint32_t total = 4 + arity * DL;
-  uint64_t a = 0;
-  for (uint32_t b0 = 0;; b0 += kc::kRateLanes) {
-    if (t < kc::kRateLanes) {
-      const uint32_t j = b0 + t;
-      uint64_t w = 0;
-      if (j < total) {
-        if (j < 4) {
-          w = j == 0 ? arity : j == 1 ? level : j == 2 ? p : label;
-        } else {
-          uint64_t c = p * arity + (j - 4) / DL;
-          if (c >= n_child) c = n_child - 1;  // padding = copies of the last node
-          w = child[DL * c + (j - 4) % DL];
-        }
-      } else if (j == total) {
-        w = 0x06ull;
-      }
-      if (t == kc::kRateLanes - 1 && b0 + kc::kRateLanes > total) w ^= 0x8000000000000000ull;
-      a ^= w;
+  const auto lane = [&](uint32_t b0) -> uint64_t {
+    if (t >= kc::kRateLanes) return 0;
+    const uint32_t j = b0 + t;
+    uint64_t w = 0;
+    if (j < 4) {
+      w = j == 0 ? arity : j == 1 ? level : j == 2 ? p : label;
+    } else if (j < total) {
+      uint64_t c = p * arity + (j - 4) / DL;
+      if (c >= n_child) c = n_child - 1;  // padding = copies of the last node
+      w = child[DL * c + (j - 4) % DL];
+    } else if (j == total) {
+      w = 0x06ull;
     }
+    if (t == kc::kRateLanes - 1 && b0 + kc::kRateLanes > total) w ^= 0x8000000000000000ull;
+    return w;
+  };
+  uint64_t a = lane(0);
+  for (uint32_t b0 = kc::kRateLanes;; b0 += kc::kRateLanes) {
+    const uint64_t w = b0 <= total ? lane(b0) : 0;  // on its way while the block before it is permuted
     keccak_f_warp(a, t);
-    if (b0 + kc::kRateLanes > total) break;
+    if (b0 > total) break;
+    a ^= w;
   }
   if (t < DL) parent[DL * p + t] = a;
 }
 
-// The levels from the first one of at most kTopWork Keccak-f (parents x
-// permutations per node: two per thread of the CTA) upward, in one CTA: each level
-// is a block-wide loop over its parents, then a barrier (which makes the level's
-// global writes visible to the whole block) before the next. Larger levels go to
-// the whole GPU: on one SM a level of 1024 arity-16 parents (4096 Keccak-f) took
-// about 0.2 ms, against a few microseconds spread over 148 SMs. Levels of at most
-// 48 parents hash each node with a warp (node_hash_warp): the tree tops of a
-// 64-byte SHA-256 proof went from 0.42 to 0.33 ms.
-constexpr int kTopThreads = 512;
-constexpr uint64_t kTopWork = 2 * kTopThreads;
-// Keccak-f per node hash: the 4-lane label and `arity` digests, padded
-inline uint64_t node_perms(uint64_t arity) { return (4 + arity * DL) / kc::kRateLanes + 1; }
+// Levels by width. Above kWarpNodes parents: a thread per node, over the whole GPU (a warp
+// a node costs some nine times the issue slots: at 28 warps an SM it is the slower one).
+// From there down: a warp per node (node_hash_warp), two warps a CTA, so that a level
+// spreads over all SMs. The last levels, of at most kTopNodes parents: one CTA, a warp per
+// node and a barrier (which makes the level's global writes visible to the whole block)
+// between the levels, which saves their launches. A node's one to five permutations are one
+// after another, about 2.5 us each with its loads, and that chain is the whole time. Up to
+// now all levels of at most 1024 permutations ran in one CTA, most by a thread a node: the
+// trees of a 64-byte SHA-256 proof took 325 us of kernel time and take 267, those of a
+// 512-point rollup 148 and 121.
+constexpr uint64_t kWarpNodes = 1024, kTopNodes = 16;
+constexpr int kTopThreads = 32 * (int)kTopNodes, kWarpNodeThreads = 64;
 constexpr int kMaxTopLevels = 24;
 struct TopLevels {
   int n;
@@ -235,30 +246,23 @@ struct TopLevels {
 __global__ void __launch_bounds__(kTopThreads) tree_top_kernel(uint64_t* d, TopLevels tl, uint64_t label,
                                                                uint64_t g_tree) {
   d += blockIdx.x * g_tree;
-  constexpr int kWarps = kTopThreads / 32;
+  const uint64_t p = threadIdx.x >> 5;
   for (int k = 0; k < tl.n; ++k) {
-    const uint64_t* ch = d + DL * tl.child_off[k];
-    uint64_t* par = d + DL * tl.parent_off[k];
-    // a narrow level (at most three nodes a warp): a warp per node, whose permutations
-    // take about a third of one thread's
-    if (tl.n_parent[k] <= 3 * kWarps) {
-      const int w = threadIdx.x >> 5, t = threadIdx.x & 31;
-      for (uint64_t p = w; p < tl.n_parent[k]; p += kWarps)
-        node_hash_warp(ch, tl.n_child[k], par, p, tl.arity[k], tl.level[k], label, t);
-      __syncthreads();
-      continue;
-    }
-    for (uint64_t p = threadIdx.x; p < tl.n_parent[k]; p += kTopThreads) {
-      switch (tl.arity[k]) {
-        case 2: node_hash<2>(ch, tl.n_child[k], par, p, tl.level[k], label); break;
-        case 4: node_hash<4>(ch, tl.n_child[k], par, p, tl.level[k], label); break;
-        case 8: node_hash<8>(ch, tl.n_child[k], par, p, tl.level[k], label); break;
-        case 16: node_hash<16>(ch, tl.n_child[k], par, p, tl.level[k], label); break;
-        default: node_hash_any(ch, tl.n_child[k], par, p, tl.arity[k], tl.level[k], label); break;
-      }
-    }
+    if (p < tl.n_parent[k])
+      node_hash_warp(d + DL * tl.child_off[k], tl.n_child[k], d + DL * tl.parent_off[k], p, tl.arity[k], tl.level[k],
+                     label, threadIdx.x & 31);
     __syncthreads();
   }
+}
+
+__global__ void __launch_bounds__(kWarpNodeThreads) node_warp_kernel(const uint64_t* child, uint64_t n_child,
+                                                                     uint64_t* parent, uint64_t n_parent,
+                                                                     uint32_t arity, uint64_t level, uint64_t label,
+                                                                     uint64_t g_tree) {
+  const uint64_t p = blockIdx.x * (uint64_t)(kWarpNodeThreads / 32) + (threadIdx.x >> 5);
+  if (p < n_parent)
+    node_hash_warp(child + blockIdx.y * g_tree, n_child, parent + blockIdx.y * g_tree, p, arity, level, label,
+                   threadIdx.x & 31);
 }
 
 __global__ void gather_digests_kernel(const uint64_t* d, const uint64_t* idx, uint64_t n, uint64_t* out) {
@@ -312,7 +316,7 @@ cudaError_t tree_hash_levels_group(const DevTree& t, uint64_t g_tree, uint32_t n
   if (n_trees == 0 || n_trees > 65535) return cudaErrorInvalidValue;
   for (size_t l = 0; l + 1 < t.len.size(); ++l) {
     const uint64_t np = t.len[l + 1];
-    if (np * node_perms(t.arity[l]) <= kTopWork && t.len.size() - 1 - l <= (size_t)kMaxTopLevels) {
+    if (np <= kTopNodes && t.len.size() - 1 - l <= (size_t)kMaxTopLevels) {
       TopLevels tl{};
       for (size_t k = l; k + 1 < t.len.size(); ++k, ++tl.n) {
         tl.arity[tl.n] = t.arity[k];
@@ -330,6 +334,12 @@ cudaError_t tree_hash_levels_group(const DevTree& t, uint64_t g_tree, uint32_t n
     uint64_t* par = t.d + DL * t.off[l + 1];
     const dim3 B(blocks_for(np, 128), n_trees);
     SG_LAUNCH_SCOPE("merkle_nodes", s);
+    if (np * n_trees <= kWarpNodes) {
+      constexpr unsigned W = kWarpNodeThreads / 32;
+      node_warp_kernel<<<dim3(blocks_for(np, W), n_trees), kWarpNodeThreads, 0, s>>>(ch, t.len[l], par, np, t.arity[l],
+                                                                                    l + 1, t.label, g_tree);
+      continue;
+    }
     switch (t.arity[l]) {
       case 2: node_kernel_t<2><<<B, 128, 0, s>>>(ch, t.len[l], par, np, l + 1, t.label, g_tree); break;
       case 4: node_kernel_t<4><<<B, 128, 0, s>>>(ch, t.len[l], par, np, l + 1, t.label, g_tree); break;
