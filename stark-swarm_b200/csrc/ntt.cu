@@ -853,7 +853,9 @@ cudaError_t ntt_batch(const NttTables& t, const uint64_t* in, uint64_t* out, uin
   }
   const uint64_t ninv = inverse ? gl::inv(N) : 1;
   const PowSpec none{};
-  if (ntt_tc_ok(log_n)) {
+  const bool apart = in + (n_cols - 1) * in_stride + N <= out || out + (n_cols - 1) * out_stride + N <= in;
+  // (2^9 points go out in two chunks, each from all inputs: not in place)
+  if (ntt_tc_ok(log_n) && (log_n != 9 || apart)) {
     TcPass p = ntt_tc_args(log_n, 0);
     p.in = in;
     p.out = out;

@@ -4,6 +4,7 @@ CTA keeps in flight, more than one chunk, both passes of a four-step transform, 
 padding, and element values whose bytes make the digit sums extreme."""
 import numpy as np
 import pytest
+import torch
 
 import oracle_lib as O
 
@@ -29,6 +30,22 @@ def test_one_pass(ctx, log_n, cols, inverse):
         got = ctx.ntt(x, log_n, inverse)
         for c in (0, cols // 2, cols - 1):
             assert np.array_equal(got[c], O.ntt(x[c], inverse)), (kind, c)
+
+
+# output over the input, with more tiles than the GPU holds at a time (a 2^9-point column
+# leaves its tile in two chunks, so the second would read what the first wrote)
+@pytest.mark.parametrize("log_n", [8, 9, 10])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_in_place(ctx, log_n, inverse):
+    x = field(np.random.default_rng(log_n), 6001, 1 << log_n)
+    d = torch.from_numpy(x.view(np.int64)).cuda()
+    torch.cuda.synchronize()
+    ctx.ntt(d, log_n, inverse, d)
+    torch.cuda.synchronize()
+    got = d.cpu().numpy().view(np.uint64)
+    assert np.array_equal(got, ctx.ntt(x, log_n, inverse))
+    for c in (0, 3000, 6000):
+        assert np.array_equal(got[c], O.ntt(x[c], inverse)), c
 
 
 # two passes: both on the tensor cores (2^16 .. 2^20), or the first one only
