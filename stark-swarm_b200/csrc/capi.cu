@@ -293,8 +293,12 @@ int sg_ntt_autotune(sg_ctx* c, size_t n_cols, size_t log_n, int inverse, size_t 
     const int prior = sg::ntt_split((int)log_n, padded);
     int best = prior;
     float best_ms = 1e30f;
+    // no split pinned goes last: it may take passes that no four-step split has, and stays
+    // unless a split is faster by more than the timing's noise
+    bool pin = true;
     try {
-      for (int l1 = lo; l1 <= hi; ++l1) {
+      for (int k = lo; k <= hi + 1; ++k) {
+        const int l1 = k <= hi ? k : 0;
         sg::ntt_set_split((int)log_n, padded, l1);
         auto run = [&] {
           sg::cuda_check(sg::ntt_batch(c->tw, in.p, out.p, (uint32_t)cols, N, N, (int)log_n, inverse != 0, n_valid,
@@ -312,7 +316,10 @@ int sg_ntt_autotune(sg_ctx* c, size_t n_cols, size_t log_n, int inverse, size_t 
           sg::cuda_check(cudaEventElapsedTime(&t, e0, e1), "elapsed");
           ms = std::min(ms, t);
         }
-        if (ms < best_ms) {
+        if (!l1) {
+          pin = best_ms < 0.98f * ms;
+          if (!pin) best = sg::ntt_split((int)log_n, padded);
+        } else if (ms < best_ms) {
           best_ms = ms;
           best = l1;
         }
@@ -323,7 +330,7 @@ int sg_ntt_autotune(sg_ctx* c, size_t n_cols, size_t log_n, int inverse, size_t 
       cudaEventDestroy(e1);
       throw;
     }
-    sg::ntt_set_split((int)log_n, padded, best);
+    sg::ntt_set_split((int)log_n, padded, pin ? best : 0);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (best_log_n1) *best_log_n1 = best;

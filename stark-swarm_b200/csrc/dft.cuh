@@ -1,8 +1,8 @@
 // dft.cuh — in-register small DFTs over Goldilocks with shift-only twiddles.
 //
 // For ark-poly's root chain the small roots are powers of two:
-// w_2 = 2^96, w_4 = 2^48, w_8 = 2^120, w_16 = 2^156 (and w_16^-1 = 2^36),
-// because 2 has order 192 in this field. A radix-R DFT (R <= 16) therefore
+// w_2 = 2^96, w_4 = 2^48, w_8 = 2^120, w_16 = 2^156 (and w_16^-1 = 2^36), w_32 = 2^78,
+// because 2 has order 192 in this field. A radix-R DFT (R <= 32) therefore
 // needs no multiplications, only shifts and 128-bit reductions.
 #pragma once
 #include "gl.cuh"
@@ -27,7 +27,8 @@ __device__ __forceinline__ void dft_reg(uint64_t* v) {
   if constexpr (R == 1) {
     return;
   } else {
-    constexpr unsigned ER = (exp16(INV) * (16 / R)) % 192;  // w_R = 2^ER
+    // w_R = 2^ER
+    constexpr unsigned ER = R == 32 ? (INV ? 114u : 78u) : (exp16(INV) * (16 / R)) % 192;
 #pragma unroll
     for (int h = R / 2; h >= 1; h >>= 1) {
 #pragma unroll

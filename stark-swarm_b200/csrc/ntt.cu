@@ -641,6 +641,96 @@ void tc_second(TcPass* p, const uint64_t* in, uint64_t* out, uint64_t out_col, i
   p->strided = true;
 }
 
+// One radix-R stage, R = 2^LR, of N = R N2 points around transforms of N2 points, N2 >= 2^8:
+// a thread per residue j < N2 and columns c = blockIdx.y, + gridDim.y, ..., with the powers of
+// X_j = g w_N^j in registers over its columns.
+//   FIRST:  out[r N2 + j] = X_j^r sum_i in[j + N2 i] w_R^(ri): the transforms of the R rows of
+//           N2 points then give the results at indices = r mod R.
+//   else:   out[j + N2 i] = sum_r w_R^(ri) X_j^r in[r N2 + j], with row r the transform of the
+//           inputs at indices = r mod R. May be in place.
+// No product but the twist's (w_R is a power of two) and no exchange between threads, and
+// both sides move in whole lines. Bound by memory (16 bytes, 2.4 ps a point) for small R, by
+// the ALU towards R = 32.
+struct RadixArgs {
+  const uint64_t* in;
+  uint64_t* out;
+  uint64_t in_col, out_col;
+  uint32_t n_cols;
+  int log_n;
+  const uint64_t *tw_lo, *tw_hi;
+  PowSpec pre;  // g (FIRST takes none)
+};
+constexpr int kRadixThreads = 128;
+
+template <int LR, bool FIRST, bool INV>
+__global__ void __launch_bounds__(kRadixThreads) radix_pass_kernel(RadixArgs a) {
+  constexpr int R = 1 << LR;
+  const uint64_t n2 = 1ull << (a.log_n - LR);
+  const uint64_t j = blockIdx.x * (uint64_t)kRadixThreads + threadIdx.x;
+  if (j >= n2) return;
+  uint64_t x[R];
+  x[1] = tw_pow(a.tw_lo, a.tw_hi, j, a.log_n);
+  if (!FIRST && a.pre.active()) x[1] = gl::mul(x[1], pow_at(a.pre, 1));
+#pragma unroll
+  for (int r = 2; r < R; ++r) x[r] = gl::mul(x[r / 2], x[r - r / 2]);
+  for (uint64_t c = blockIdx.y; c < a.n_cols; c += gridDim.y) {
+    const uint64_t* in = a.in + c * a.in_col + j;
+    uint64_t* out = a.out + c * a.out_col + j;
+    uint64_t v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = in[r * n2];
+    if constexpr (!FIRST) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = gl::mul(v[r], x[r]);
+    }
+    dft_reg<R, INV>(v);
+    if constexpr (FIRST) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = gl::mul(v[r], x[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) out[r * n2] = v[r];
+  }
+}
+
+template <int LR>
+cudaError_t radix_launch(const RadixArgs& a, bool first, bool inv, cudaStream_t s) {
+  const uint64_t n2 = 1ull << (a.log_n - LR), bx = (n2 + kRadixThreads - 1) / kRadixThreads;
+  // columns share their thread's powers once there are some four waves of CTAs
+  const uint64_t by = std::min<uint64_t>(std::min<uint64_t>(a.n_cols, 65535), std::max<uint64_t>(1, 148 * 16 / bx));
+  const dim3 grid((unsigned)bx, (unsigned)by);
+  SG_LAUNCH_SCOPE("ntt_radix", s);
+  if (first)
+    radix_pass_kernel<LR, true, true><<<grid, kRadixThreads, 0, s>>>(a);
+  else if (inv)
+    radix_pass_kernel<LR, false, true><<<grid, kRadixThreads, 0, s>>>(a);
+  else
+    radix_pass_kernel<LR, false, false><<<grid, kRadixThreads, 0, s>>>(a);
+  return cudaGetLastError();
+}
+cudaError_t radix_pass(int lr, const RadixArgs& a, bool first, bool inv, cudaStream_t s) {
+  switch (lr) {
+    case 1: return radix_launch<1>(a, first, inv, s);
+    case 2: return radix_launch<2>(a, first, inv, s);
+    case 3: return radix_launch<3>(a, first, inv, s);
+    case 4: return radix_launch<4>(a, first, inv, s);
+    case 5: return radix_launch<5>(a, first, inv, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+RadixArgs radix_args(const NttTables& t, const uint64_t* in, uint64_t in_col, uint64_t* out, uint64_t out_col,
+                     uint32_t n_cols, int log_n, bool inverse) {
+  return RadixArgs{in, out, in_col, out_col, n_cols, log_n, inverse ? t.d_inv_lo : t.d_fwd_lo,
+                   inverse ? t.d_inv_hi : t.d_fwd_hi, {}};
+}
+
+// 2^11 .. 2^15 points: too many for one tensor-core pass (2^10), too few for two (2^16), so
+// that one or both passes were shared-memory ones. With a radix stage instead, LDE: 1000 x
+// 2^11 x 32 1010 -> 489 us, 500 x 2^12 x 32 1129 -> 515, 64 x 2^13 x 32 244 -> 168, 256 x 2^14
+// x 16 869 -> 600, 64 x 2^15 x 32 969 -> 648, 3 x 2^11 x 32 62 -> 45; one transform: 2000 x
+// 2^11 71 -> 55, 64 x 2^12 45 -> 27, 3000 x 2^13 470 -> 239, 1000 x 2^15 472 -> 399 us.
+bool radix_size(int log_n) { return log_n >= 11 && log_n <= 15; }
+
 int sparse_nz_for(uint64_t n_valid, uint64_t N, uint64_t n_lo, uint64_t M) {
   if (n_valid >= N || M < 16) return 0;  // dense, or a pass without a radix-16 first stage
   const uint64_t m_nz = (n_valid + n_lo - 1) / n_lo, G = M / 16;
@@ -725,7 +815,8 @@ void ntt_tables_free(NttTables* t) {
 }
 
 bool ntt_coset_eval_ok(int log_m, int log_b) {
-  return log_m >= 1 && log_m <= 12 && (ntt_tc_ok(log_m) || log_b >= pass_log_k(log_m)) && log_m + log_b <= kMaxLogN;
+  return log_m >= 1 && log_m <= 12 && log_m + log_b <= kMaxLogN &&
+         (ntt_tc_ok(std::max(log_m, 8)) ? log_m + log_b >= 8 : log_b >= pass_log_k(log_m));
 }
 
 // Coset t < B of the evaluation domain is the DFT_M of c_m * g^m * w_N^{t m}:
@@ -738,8 +829,10 @@ cudaError_t ntt_coset_eval(const NttTables& t, const uint64_t* coef, uint64_t* o
   if (!ntt_coset_eval_ok(log_m, log_b)) return cudaErrorInvalidValue;
   if (n_cols == 0) return cudaSuccess;
   const uint64_t M = 1ull << log_m, B = 1ull << log_b;
-  if (ntt_tc_ok(log_m)) {
-    TcPass p = ntt_tc_args(log_m, log_b);
+  // fewer than 2^8 coefficients: as 2^8, zero-padded
+  const int lm = std::max(log_m, 8), le = log_m + log_b - lm;
+  if (ntt_tc_ok(lm) && le >= 0) {
+    TcPass p = ntt_tc_args(lm, le);
     p.in = coef;
     p.out = out;
     p.in_lane = M;
@@ -868,6 +961,37 @@ cudaError_t ntt_batch(const NttTables& t, const uint64_t* in, uint64_t* out, uin
     p.pre = pre ? *pre : none;
     p.scale = ninv;
     if (ntt_tc_tables(t, &p, inverse, s)) return ntt_tc_pass(p, false, s);
+  }
+  if (radix_size(log_n) && n_valid == N && (apart || (scratch && log_n > 12)) && !g_split[log_n][0].load()) {
+    // the R interleaved transforms of 2^10 points (2^8 for 2^11, whose eight lanes fill a
+    // tile), then the radix-R stage, in place unless the input is there
+    const int lm = log_n == 11 ? 8 : 10, lr = log_n - lm;
+    const uint64_t R = 1ull << lr;
+    uint64_t* mid = apart ? out : scratch;
+    const uint64_t mid_col = apart ? out_stride : N;
+    TcPass p = ntt_tc_args(lm, 0);
+    p.in = in;
+    p.out = mid;
+    p.in_col = in_stride;
+    p.out_col = mid_col;
+    p.in_lane = 1;
+    p.in_m = R;
+    p.out_lane = N >> lr;
+    tc_out(&p, 1);
+    p.n_lanes = (uint32_t)R;
+    p.n_y = n_cols;
+    p.flat_m = R;
+    p.in_valid = N;
+    p.pre = pre ? *pre : none;
+    p.scale = ninv;
+    p.strided = true;
+    if (ntt_tc_tables(t, &p, inverse, s)) {
+      const cudaError_t e = ntt_tc_pass(p, true, s);
+      if (e != cudaSuccess) return e;
+      RadixArgs a = radix_args(t, mid, mid_col, out, out_stride, n_cols, log_n, inverse);
+      if (pre) a.pre = *pre;
+      return radix_pass(lr, a, false, inverse, s);
+    }
   }
   if (log_n <= 12) {
     // one pass; the lanes are the columns (a length-1 "transform" is the identity
@@ -1020,10 +1144,57 @@ cudaError_t ntt_batch(const NttTables& t, const uint64_t* in, uint64_t* out, uin
   return launch_pass_dyn(la, c, inverse, n_cols, s);
 }
 
+// An LDE of 2^11 .. 2^15 rows: each row index k = R k2 + r splits into R = 2^(log_n - 10)
+// interleaved parts f_r of 2^10 coefficients, f(X) = sum_r X^r f_r(X^R). The inverse's radix
+// stage comes first and leaves the parts' coefficients apart, one tensor-core pass evaluates
+// all parts on the coset (of g^R, blowup 2^log_b), and the forward radix stage joins them in
+// place: two light passes in place of a second transform, and no scratch.
+static cudaError_t lde_radix(const NttTables& t, const uint64_t* in, uint64_t* coef, uint64_t* out, uint32_t n_cols,
+                             int log_n, int log_b, cudaStream_t s, const PowSpec* pre) {
+  constexpr int LM = 10;
+  const int lr = log_n - LM, log_e = log_n + log_b;
+  const uint64_t n = 1ull << log_n, M = 1ull << LM;
+  if (log_e > kMaxLogN || (uint64_t)n_cols << lr > 0x7FFFFFFFull) return cudaErrorNotSupported;
+  TcPass p[2] = {ntt_tc_args(LM, 0), ntt_tc_args(LM, log_b)};
+  for (TcPass& q : p) {
+    q.in = coef;
+    q.in_lane = M;
+    q.in_m = 1;
+    q.n_lanes = n_cols << lr;
+    q.in_valid = n;
+    tc_out(&q, 1);
+  }
+  p[0].out = coef;  // in place: a tile holds its lanes whole
+  p[0].out_lane = M;
+  p[0].scale = gl::inv(n);
+  p[1].out = out;
+  p[1].out_lane = M << log_b;
+  p[1].flat_m = 1ull << lr;
+  if (pre) p[1].pre = *pre;
+  if (!ntt_tc_tables(t, &p[0], true, s)) return cudaErrorNotSupported;
+  if (!ntt_tc_tables(t, &p[1], false, s)) {
+    ntt_tc_drop(p[0], s);
+    return cudaErrorNotSupported;
+  }
+  cudaError_t e = radix_pass(lr, radix_args(t, in, n, coef, n, n_cols, log_n, true), true, true, s);
+  for (const TcPass& q : p) {
+    if (e == cudaSuccess)
+      e = ntt_tc_pass(q, false, s);
+    else
+      ntt_tc_drop(q, s);
+  }
+  if (e != cudaSuccess) return e;
+  RadixArgs a = radix_args(t, out, n << log_b, out, n << log_b, n_cols, log_e, false);
+  if (pre) a.pre = *pre;
+  return radix_pass(lr, a, false, false, s);
+}
+
 // Inverse transform and zero-padded forward transform with the coefficients between them
 // in blocks (tc_first's and tc_second's): both ends of that buffer then move whole pieces.
 cudaError_t ntt_lde(const NttTables& t, const uint64_t* in, uint64_t* coef, uint64_t* out, uint32_t n_cols, int log_n,
                     int log_b, uint64_t* scratch, cudaStream_t s, const PowSpec* pre) {
+  if (t.tc && radix_size(log_n) && log_b >= 1 && n_cols > 0)
+    return lde_radix(t, in, coef, out, n_cols, log_n, log_b, s, pre);
   const int log_e = log_n + log_b, l1 = log_n / 2, l2 = log_n - l1;
   if (!t.tc || !ntt_tc_ok(l1) || !ntt_tc_ok(l2) || log_b < 1 || log_e > 24 || !scratch || n_cols == 0 ||
       g_split[log_n][0].load() || g_split[log_e][1].load())

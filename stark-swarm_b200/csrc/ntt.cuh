@@ -88,9 +88,10 @@ cudaError_t ntt_batch(const NttTables& t, const uint64_t* in, uint64_t* out, uin
 
 // The LDE of n_cols columns of 2^log_n values (column stride 2^log_n) onto 2^(log_n + log_b)
 // points, as ntt_batch's inverse and then its zero-padded forward transform with `pre`, for
-// traces of 2^16 .. 2^20 rows; coef (n_cols 2^log_n elements) holds the coefficients in an
+// traces of 2^11 .. 2^20 rows; coef (n_cols 2^log_n elements) holds the coefficients in an
 // order of its own. cudaErrorNotSupported (nothing done) when these transforms do not run
-// on the tensor cores or a split is pinned. scratch: ntt_scratch_elems(n_cols, log_n + log_b).
+// on the tensor cores or, from 2^16 rows, a split is pinned.
+// scratch (from 2^16 rows): ntt_scratch_elems(n_cols, log_n + log_b).
 cudaError_t ntt_lde(const NttTables& t, const uint64_t* in, uint64_t* coef, uint64_t* out, uint32_t n_cols, int log_n,
                     int log_b, uint64_t* scratch, cudaStream_t s, const PowSpec* pre = nullptr);
 
@@ -98,8 +99,8 @@ cudaError_t ntt_lde(const NttTables& t, const uint64_t* in, uint64_t* coef, uint
 // column stride M) on the N = M * 2^log_b points g * w_N^j in natural order
 // (column stride N) in one pass, without scratch: a forward transform of the
 // zero-padded coefficients times g^k, as ntt_batch computes it with `pre`.
-// Needs ntt_coset_eval_ok(log_m, log_b): log_m <= 12 and at least as many
-// cosets as a pass's lanes per CTA.
+// Needs ntt_coset_eval_ok(log_m, log_b): log_m <= 10 and N >= 2^8, or log_m <= 12 and at
+// least as many cosets as a pass's lanes per CTA.
 bool ntt_coset_eval_ok(int log_m, int log_b);
 cudaError_t ntt_coset_eval(const NttTables& t, const uint64_t* coef, uint64_t* out, uint32_t n_cols, int log_m,
                            int log_b, cudaStream_t s, const PowSpec* pre = nullptr);

@@ -84,10 +84,12 @@ struct ShiftTables {
 
 // A domain above one pass (2^12) from a trace of at most 2^12 rows is evaluated
 // coset by coset in one pass (ntt_coset_eval): no scratch round trip, and no
-// scratch buffer the size of the LDE.
+// scratch buffer the size of the LDE. Traces of fewer than 2^8 rows go there from
+// 2^11 points, where the transform of the padded coefficients would leave the tensor
+// cores (2000 x 2^7 x 32: 163 us, so 77).
 bool lde_by_cosets(uint64_t n_trace, uint64_t blowup) {
   const int lm = (int)log2_exact(n_trace), lb = (int)log2_exact(blowup);
-  return (lm + lb > 12 || ntt_tc_ok(lm)) && ntt_coset_eval_ok(lm, lb);
+  return (lm + lb > 12 || ntt_tc_ok(lm) || (lm < 8 && lm + lb > 10)) && ntt_coset_eval_ok(lm, lb);
 }
 
 // iNTT of w columns into coef, then the zero-padded forward transform into d_out,

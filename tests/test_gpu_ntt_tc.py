@@ -48,6 +48,36 @@ def test_in_place(ctx, log_n, inverse):
         assert np.array_equal(got[c], O.ntt(x[c], inverse)), c
 
 
+# 2^11 .. 2^15 points: interleaved transforms and a radix stage (columns that share a
+# thread's powers in the stage's loop and a last ragged turn, one column, in place)
+@pytest.mark.parametrize("log_n,cols", [(11, 1), (11, 1200), (12, 1), (12, 301), (13, 2), (13, 160), (14, 1), (14, 75), (15, 3),
+                                        (15, 40)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_radix_stage(ctx, log_n, cols, inverse):
+    x = field(np.random.default_rng(log_n + cols), cols, 1 << log_n, "extreme" if cols == 1 else "random")
+    got = ctx.ntt(x, log_n, inverse)
+    for c in (0, cols // 2, cols - 1):
+        assert np.array_equal(got[c], O.ntt(x[c], inverse)), c
+    d = torch.from_numpy(x.view(np.int64)).cuda()
+    torch.cuda.synchronize()
+    ctx.ntt(d, log_n, inverse, d)
+    torch.cuda.synchronize()
+    assert np.array_equal(d.cpu().numpy().view(np.uint64), got)
+
+
+# LDE of fewer than 2^8 rows as zero-padded cosets, and of 2^11 .. 2^15 rows in interleaved
+# parts joined by a radix stage
+@pytest.mark.parametrize("w,log_n,blowup,shift", [
+    (3, 3, 256, 7), (1, 4, 128, 1), (9, 5, 64, 5), (2, 6, 32, 1), (17, 6, 64, 7), (5, 7, 16, 1), (33, 7, 32, 7), (1, 7, 256, 3),
+    (1, 11, 2, 7), (301, 11, 8, 1), (7, 11, 32, 3), (2, 12, 2, 1), (75, 12, 32, 7), (1, 13, 4, 7), (3, 13, 32, 1), (2, 14, 2, 5),
+    (5, 14, 16, 1), (1, 15, 2, 1), (3, 15, 32, 7),
+])
+def test_lde_radix_and_short(ctx, w, log_n, blowup, shift):
+    tr = field(np.random.default_rng(w + 10 * log_n), w, 1 << log_n, "extreme" if w == 2 else "random")
+    pick = [0, w // 2, w - 1]
+    assert np.array_equal(ctx.lde(tr, blowup, shift)[pick], O.lde(np.ascontiguousarray(tr[pick]), blowup, shift))
+
+
 # two passes: both on the tensor cores (2^16 .. 2^20), or the first one only
 @pytest.mark.parametrize("log_n,cols", [(13, 3), (14, 1), (15, 2), (16, 1), (16, 5), (17, 2), (18, 1), (19, 3), (20, 1),
                                         (21, 1), (22, 1)])
