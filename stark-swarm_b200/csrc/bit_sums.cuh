@@ -13,12 +13,13 @@
 namespace sg {
 namespace bsum {
 
-// lam u + e for lam < 2^18, any u and e < 2^63, as some u64 of its residue class
+// lam u + e for any u, as some u64 of its residue class; (lam + 1) 2^32 + e at most 2^64 (so
+// lam < 2^18 and e < 2^63, or any lam and e = 0)
 __device__ __forceinline__ uint64_t mul18_add(uint32_t lam, uint64_t u, uint64_t e) {
   const uint64_t w = (uint64_t)lam * (uint32_t)u + e;
   const uint64_t v = (uint64_t)lam * (uint32_t)(u >> 32) + (w >> 32);
   uint64_t r;
-  // (v : low word of w) with the word h above 2^64 (below 2^19) folded: + h 2^32 - h
+  // (v : low word of w) with the word h above 2^64 folded: + h 2^32 - h
   asm("{\n\t.reg .u32 w0, w1, v0, h, t, lo, hi;\n\tmov.b64 {w0, w1}, %1;\n\tmov.b64 {v0, h}, %2;\n\t"
       "add.cc.u32 t, v0, h;\n\taddc.u32 h, h, 0;\n\tadd.u32 hi, v0, h;\n\t"
       "sub.cc.u32 lo, w0, h;\n\tsubc.u32 hi, hi, 0;\n\tmov.b64 %0, {lo, hi};\n\t}"

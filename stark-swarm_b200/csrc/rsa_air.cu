@@ -6,10 +6,17 @@
 // Phi layout: one CTA per (4 consecutive LDE points, record). The 4 points are
 // one 32-byte sector of every column, so each cell load of the CTA is one
 // sector for 4 threads; the points share their trace row (blowup >= 4). The
-// limbs the slot identities convolve (acc, op2, q, n, c) and the 158 signed
-// carries are staged in shared memory; every other constraint reads its cells
-// directly. Each thread accumulates lambda_j C_j for one point; a warp shuffle
-// and a shared-memory pass reduce the 256 partial sums to the 4 points.
+// limbs the slot identities convolve (acc, op2, q, n, c) are staged in shared
+// memory; every other constraint reads its cells directly. Each thread
+// accumulates lambda_j C_j for one point in unreduced sums; a warp shuffle and a
+// shared-memory pass reduce the 256 partial sums to the 4 points.
+//
+// Bound by the latency of those sectors (92 MB a record, a column every 8 KB at 1024
+// points). With a thread per limb or carry, whose bits it read in turn, the CTA's loads were
+// spread over 20 MB and a record took 112 us, unreduced sums or not; as products that need
+// no order, each step of the CTA takes 64 adjacent columns: 65 us. 512 threads a CTA: 63 us
+// for one record, no gain for many.
+#include "bit_sums.cuh"
 #include "context.hpp"
 #include "counters.hpp"
 #include "gl.cuh"
@@ -32,19 +39,6 @@ __global__ void rsa_expand_kernel(const RecordW* recs, const RowW* rows, uint64_
   }
 }
 
-// lambda C summed in a field accumulator
-struct Acc {
-  uint64_t v = 0;
-  __device__ __forceinline__ void put(uint64_t lambda, uint64_t c) { v = gl::add(v, gl::mul(lambda, c)); }
-};
-
-// sum_b 2^b x_b for b < nb (Horner from the top bit), over field cells
-__device__ __forceinline__ uint64_t pack_bits(const uint64_t* col0, uint64_t n, uint32_t nb) {
-  uint64_t s = 0;
-  for (int b = (int)nb - 1; b >= 0; --b) s = gl::add(gl::add(s, s), __ldg(col0 + (uint64_t)b * n));
-  return s;
-}
-
 __global__ void __launch_bounds__(kThreads) rsa_phi_kernel(const uint64_t* lde, uint64_t n, uint64_t blowup,
                                                            uint64_t n_trace, uint64_t* phi_part) {
   const uint64_t i0 = (uint64_t)blockIdx.x * kPts, rec = blockIdx.y;
@@ -58,7 +52,6 @@ __global__ void __launch_bounds__(kThreads) rsa_phi_kernel(const uint64_t* lde, 
   auto nxt = [&](uint32_t col) { return __ldg(L + (uint64_t)col * n + nx0 + p); };
 
   __shared__ uint64_t sa[LIMBS][kPts], sb[LIMBS][kPts], sq[LIMBS][kPts], sn[LIMBS][kPts], sc[LIMBS][kPts];
-  __shared__ uint64_t sk[CARRY_POS][kPts];  // signed carries sum_b 2^b bit - 2^39
   for (int e = t; e < (int)(LIMBS * kPts); e += kThreads) {
     const int i = e / kPts;
     sa[i][p] = cur(ACC + i);
@@ -67,65 +60,78 @@ __global__ void __launch_bounds__(kThreads) rsa_phi_kernel(const uint64_t* lde, 
     sn[i][p] = cur(N + i);
     sc[i][p] = cur(C + i);
   }
-  for (int e = t; e < (int)(CARRY_POS * kPts); e += kThreads) {
-    const int k = e / kPts;
-    sk[k][p] = gl::sub(pack_bits(L + (uint64_t)(CARRY + k * CARRY_BITS) * n + i0 + p, n, CARRY_BITS),
-                       CARRY_OFFSET);
+
+  gl::AccProd acc, neg;  // Phi = acc - neg
+  auto put = [&](uint64_t lambda, uint64_t c) { acc.add(c, lambda); };
+  // Nine tenths of the cells are bits, and Phi is linear in the sums that they stand for: a
+  // bit's booleanity and its part of a limb or carry are one product t (lambda (t - 1) + w),
+  // taken off. So the bits need no order: a step takes 64 adjacent columns.
+  auto bits = [&](uint32_t col, int count, auto weight) {
+    constexpr int U = 8, S = kThreads / kPts;
+    for (int j = t / kPts; j < count; j += U * S) {
+      uint64_t x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) x[u] = j + u * S < count ? cur(col + j + u * S) : 0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) neg.add(x[u], weight((uint32_t)(j + u * S), x[u]));
+    }
+  };
+  const uint32_t lam32 = (uint32_t)lam0;  // below 2^30 for 65535 records
+  // limb bits: w = lambda_pack 2^b, from limb - sum_b 2^b t_b
+  auto limb_bits = [&](uint32_t col, uint32_t k_bool, uint32_t k_pack) {
+    bits(col, LIMBS * LIMB_BITS, [=](uint32_t j, uint64_t x) {
+      const uint32_t lam = lam32 + k_bool + j;
+      return bsum::mul18_add(lam, x, ((uint64_t)(lam32 + k_pack + j / LIMB_BITS) << (j % LIMB_BITS)) - lam);
+    });
+  };
+  limb_bits(C_BITS, K_CBOOL, K_CPACK);
+  limb_bits(Q_BITS, K_QBOOL, K_QPACK);
+  // carry bits: slot k + 1 adds carry k = sum_b 2^b t_b - 2^39 and slot k takes 2^26 times it
+  // off, so w = D_k 2^b with D_k = 2^26 lambda_k - lambda_(k+1), and D_k 2^39 stays
+  bits(CARRY, CARRY_POS * CARRY_BITS, [=](uint32_t j, uint64_t x) {
+    const uint32_t k = j / CARRY_BITS, b = j % CARRY_BITS, lam_k = lam32 + K_SLOT + k;
+    const uint64_t d = ((uint64_t)lam_k << LIMB_BITS) - (lam_k + 1);
+    return gl::add(bsum::mul18_add(lam32 + K_CARRY + j, gl::sub(x, 1), 0),
+                   gl::reduce128(d >> 1 >> (63 - b), d << b));
+  });
+  if (t < kPts) {
+    constexpr uint64_t n_c = CARRY_POS;
+    const uint64_t lam_sum = n_c * (lam0 + K_SLOT) + n_c * (n_c - 1) / 2;
+    put((lam_sum << LIMB_BITS) - (lam_sum + n_c), CARRY_OFFSET);
   }
   __syncthreads();
+  for (int e = t; e < (int)(2 * LIMBS * kPts); e += kThreads) {
+    const int j = e / kPts, i = j < (int)LIMBS ? j : j - (int)LIMBS;
+    put(lam0 + (j < (int)LIMBS ? K_CPACK : K_QPACK) + i, (j < (int)LIMBS ? sc : sq)[i][p]);
+  }
 
-  Acc acc;
   const uint64_t phase = cur(PHASE);
-  if (t < kPts) acc.put(lam0 + K_PHASE, gl::mul(phase, gl::sub(1, phase)));
+  if (t < kPts) put(lam0 + K_PHASE, gl::mul(phase, gl::sub(1, phase)));
   // select
   for (int e = t; e < (int)(LIMBS * kPts); e += kThreads) {
     const int i = e / kPts;
     const uint64_t a = sa[i][p];
     const uint64_t target = gl::add(gl::mul(phase, gl::sub(cur(S + i), a)), a);
-    acc.put(lam0 + K_SELECT + i, gl::sub(sb[i][p], target));
+    put(lam0 + K_SELECT + i, gl::sub(sb[i][p], target));
   }
-  // booleanity of the c bits, q bits and carry bits
-  for (int e = t; e < (int)(2 * LIMBS * LIMB_BITS * kPts); e += kThreads) {
-    const int j = e / kPts;  // 0 .. 4159: c bits then q bits
-    const bool is_c = j < (int)(LIMBS * LIMB_BITS);
-    const uint32_t off = is_c ? j : j - LIMBS * LIMB_BITS;
-    const uint64_t x = cur((is_c ? C_BITS : Q_BITS) + off);
-    acc.put(lam0 + (is_c ? K_CBOOL : K_QBOOL) + off, gl::mul(x, gl::sub(1, x)));
-  }
-  for (int e = t; e < (int)(CARRY_POS * CARRY_BITS * kPts); e += kThreads) {
-    const int j = e / kPts;
-    const uint64_t x = cur(CARRY + j);
-    acc.put(lam0 + K_CARRY + j, gl::mul(x, gl::sub(1, x)));
-  }
-  // limb packs
-  for (int e = t; e < (int)(2 * LIMBS * kPts); e += kThreads) {
-    const int j = e / kPts;
-    const bool is_c = j < (int)LIMBS;
-    const int i = is_c ? j : j - LIMBS;
-    const uint64_t bits = pack_bits(L + (uint64_t)((is_c ? C_BITS : Q_BITS) + i * LIMB_BITS) * n + i0 + p, n,
-                                    LIMB_BITS);
-    acc.put(lam0 + (is_c ? K_CPACK : K_QPACK) + i, gl::sub(is_c ? sc[i][p] : sq[i][p], bits));
-  }
-  // slot identities: sum a_i b_{k-i} - sum q_i n_{k-i} - c_k + carry_{k-1} - 2^26 carry_k
+  // slot identities: sum a_i b_{k-i} - sum q_i n_{k-i} - c_k (+ carry_{k-1} - 2^26 carry_k, above)
   for (int e = t; e < (int)(SLOTS * kPts); e += kThreads) {
     const int k = e / kPts;
     const int lo = k >= (int)LIMBS - 1 ? k - (int)(LIMBS - 1) : 0, hi = k < (int)LIMBS - 1 ? k : LIMBS - 1;
-    uint64_t ab = 0, qn = 0;
+    gl::AccProd ab, qn;
     for (int i = lo; i <= hi; ++i) {
-      ab = gl::add(ab, gl::mul(sa[i][p], sb[k - i][p]));
-      qn = gl::add(qn, gl::mul(sq[i][p], sn[k - i][p]));
+      ab.add(sa[i][p], sb[k - i][p]);
+      qn.add(sq[i][p], sn[k - i][p]);
     }
-    uint64_t v = gl::sub(ab, qn);
+    uint64_t v = gl::sub(ab.reduce(), qn.reduce());
     if (k < (int)LIMBS) v = gl::sub(v, sc[k][p]);
-    if (k > 0) v = gl::add(v, sk[k - 1][p]);
-    if (k < (int)CARRY_POS) v = gl::sub(v, gl::mul_pow2(sk[k][p], LIMB_BITS));
-    acc.put(lam0 + K_SLOT + k, v);
+    put(lam0 + K_SLOT + k, v);
   }
   // row-16 boundary and the transitions (zero elsewhere: no contribution)
   if (out_row)
     for (int e = t; e < (int)(LIMBS * kPts); e += kThreads) {
       const int i = e / kPts;
-      acc.put(lam0 + K_EM + i, gl::sub(sc[i][p], cur(EM + i)));
+      put(lam0 + K_EM + i, gl::sub(sc[i][p], cur(EM + i)));
     }
   if (trans)
     for (int e = t; e < (int)(4 * LIMBS * kPts); e += kThreads) {
@@ -137,11 +143,11 @@ __global__ void __launch_bounds__(kThreads) rsa_phi_kernel(const uint64_t* lde, 
         const uint32_t col = (g == 1 ? S : g == 2 ? N : EM) + i;
         v = gl::sub(nxt(col), cur(col));
       }
-      acc.put(lam0 + K_TRANS + j, v);
+      put(lam0 + K_TRANS + j, v);
     }
 
   // reduce the threads of each point: lanes l, l + 4, ... share a point
-  uint64_t v = acc.v;
+  uint64_t v = gl::sub(acc.reduce(), neg.reduce());
 #pragma unroll
   for (int o = 16; o >= kPts; o >>= 1) v = gl::add(v, __shfl_down_sync(0xffffffffu, v, o));
   __shared__ uint64_t red[kThreads / 32][kPts];
