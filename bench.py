@@ -145,18 +145,19 @@ class ClockSampler:
                 "samples": len(sm)}
 
 
-# Integer-pipe roofline and DRAM traffic of the dominant kernels, from ncu on the
-# reduced case (4 columns, 2^20 -> 2^23; 256 MiB LDE, larger than L2), scaled to 64
-# columns by the columns processed. int_frac = ALU-pipe instructions issued / peak
-# over the kernel's active cycles (sm__inst_executed_pipe_alu.avg.pct_of_peak_
-# sustained_active): these kernels are bound by integer issue, not by HBM.
-#   ntt_pass <12,fwd> 500.6 us: ALU 64.2 %, DRAM 0.498 TB/s -> 249 MB per 4 columns
-#   ntt_pass <11,fwd> 386.1 us: ALU 64.2 %, DRAM 1.275 TB/s -> 492 MB per 4 columns
-#   ntt_pass <10,inv> x 2 (trace iNTT, 16-column capture): 471 MB per 16 columns
-#   leaf_kernel_t<64> (2^20 rows of 64 columns) 1.489 ms: ALU 83.2 %
-_LDE_TRAFFIC = (249e6 + 492e6) * 16 + 471e6 * 4  # bytes per 64-column LDE (4 launches)
+# Pipe shares and DRAM traffic of the dominant kernels, from ncu on reduced cases, the
+# traffic scaled to 64 columns by the columns processed. int_frac = ALU-pipe share of the
+# kernel's active cycles (sm__pipe_alu_cycles_active), over a transform's launches by time.
+# 16 columns, 2^20 -> 2^23 (1 GiB LDE), the four tensor-core passes:
+#   inverse 2^20, pass 1: 168.9 us, 225 MB; pass 2: 87.8 us, 221 MB
+#   forward 2^23, pass 1: 827 us, 2.11 GB: ALU 42 %, FMA 52 %, tensor 31 %
+#   forward 2^23, pass 2: 753 us, 2.10 GB: ALU 33 %, FMA 40 %, tensor 34 %
+# leaf_kernel_t<64> (2^20 rows of 64 columns): ALU 83.2 % at 1.489 ms, before its rounds
+# were rolled (1.405 ms)
+_LDE_TRAFFIC = (225e6 + 221e6 + 2.11e9 + 2.10e9) * 4  # bytes per 64-column LDE (4 launches)
 MEASURED_NTT = {
-    "ntt_pass": {"int_frac": 0.642, "int_metric": "ALU-pipe share of active cycles (ncu, 4-column case)",
+    "ntt_pass": {"int_frac": 0.38, "int_metric": "ALU-pipe share of active cycles (ncu, 16-column case); FMA pipe 0.46, "
+                                                 "tensor pipe 0.33",
                  "traffic_per_lde": _LDE_TRAFFIC},
     "merkle_leaves": {"int_frac": 0.832, "int_metric": "ALU-pipe share of active cycles (ncu, 2^20 x 64 leaves)"},
 }

@@ -1,5 +1,10 @@
 // ntt.cu — batched Goldilocks NTT for sm_100a.
 //
+// Passes of 2^8 .. 2^10 points run on the tensor cores (ntt_tc.cu) where the tables have
+// their cache: sizes 2^8 .. 2^10 as one such pass, 2^11 .. 2^15 as interleaved ones and a
+// radix stage, 2^16 .. 2^20 as two. What follows describes the other sizes, calls that must not
+// allocate, and the splits.
+//
 // Global structure: a transform of N = 2^n <= 2^12 is one pass; up to 2^24 it
 // is a four-step split N = N1 * N2 (N1 <= N2 <= 2^12) done as two passes:
 //   pass 1: for each k1 < N1, DFT_{N2} over k2 of x[k2*N1 + k1], times w_N^{i2*k1},

@@ -66,12 +66,12 @@ uint64_t footprint_bytes(const sg_job& j) {
   if (j.kind == SG_JOB_SHA256) {
     const uint64_t blocks = (j.input_len + 9 + 63) / 64;
     const uint64_t nt = next_pow2(128 * blocks), n0 = nt * bu;
-    return 8 * ((uint64_t)sg::sha::WIDTH * (n0 + 2 * nt) + 16 * n0);
+    return 8 * ((uint64_t)sg::sha::WIDTH * (n0 + 2 * nt) + (16 + 16) * n0);  // Phi's partial sums among them
   }
   if (j.kind == SG_JOB_SHA512) {
     const uint64_t blocks = (j.input_len + 17 + 127) / 128;
     const uint64_t nt = next_pow2(128 * blocks), n0 = nt * bu;
-    return 8 * ((uint64_t)sg::sha512::WIDTH * (n0 + 2 * nt) + 16 * n0);
+    return 8 * ((uint64_t)sg::sha512::WIDTH * (n0 + 2 * nt) + (16 + 39) * n0);
   }
   if (j.kind == SG_JOB_P256_ECDSA) {
     // trace, coefficients and LDE at 151,334 columns (the LDE is evaluated
