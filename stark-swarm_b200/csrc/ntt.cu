@@ -729,6 +729,37 @@ RadixArgs radix_args(const NttTables& t, const uint64_t* in, uint64_t in_col, ui
                    inverse ? t.d_inv_hi : t.d_fwd_hi, {}};
 }
 
+// A transform of 2 .. 32 points by one thread: a thread a column, no twiddle and no exchange.
+// A launch of few columns is bound by its latency: a call of 6 x 2^4 takes 13 us where the
+// shared-memory pass took 19, 11041 x 2^5 (an RSA trace) 19.6 and 21.4. Each thread walks its
+// own lines, so the gain goes with the columns (40000 x 2^4: 19.2 and 20.1); above kTinyCols
+// the pass that loads whole tiles stays.
+constexpr uint32_t kTinyCols = 32768;
+template <int LR, bool INV>
+__global__ void __launch_bounds__(32) tiny_ntt_kernel(const uint64_t* in, uint64_t* out, uint64_t in_stride,
+                                                      uint64_t out_stride, uint32_t n_cols, uint32_t n_valid) {
+  constexpr int R = 1 << LR;
+  const uint32_t c = blockIdx.x * 32 + threadIdx.x;
+  if (c >= n_cols) return;
+  uint64_t v[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] = r < n_valid ? in[c * in_stride + r] : 0;
+  dft_reg<R, INV>(v);
+#pragma unroll
+  for (int r = 0; r < R; ++r) out[c * out_stride + r] = INV ? gl::mul_pow2(v[r], 192 - LR) : v[r];
+}
+template <int LR>
+cudaError_t tiny_ntt(const uint64_t* in, uint64_t* out, uint64_t in_stride, uint64_t out_stride, uint32_t n_cols,
+                     uint32_t n_valid, bool inv, cudaStream_t s) {
+  SG_LAUNCH_SCOPE("ntt_radix", s);
+  const unsigned blocks = (n_cols + 31) / 32;
+  if (inv)
+    tiny_ntt_kernel<LR, true><<<blocks, 32, 0, s>>>(in, out, in_stride, out_stride, n_cols, n_valid);
+  else
+    tiny_ntt_kernel<LR, false><<<blocks, 32, 0, s>>>(in, out, in_stride, out_stride, n_cols, n_valid);
+  return cudaGetLastError();
+}
+
 // 2^11 .. 2^15 points: too many for one tensor-core pass (2^10), too few for two (2^16), so
 // that one or both passes were shared-memory ones. With a radix stage instead, LDE: 1000 x
 // 2^11 x 32 1010 -> 489 us, 500 x 2^12 x 32 1129 -> 515, 64 x 2^13 x 32 244 -> 168, 256 x 2^14
@@ -996,6 +1027,16 @@ cudaError_t ntt_batch(const NttTables& t, const uint64_t* in, uint64_t* out, uin
       RadixArgs a = radix_args(t, mid, mid_col, out, out_stride, n_cols, log_n, inverse);
       if (pre) a.pre = *pre;
       return radix_pass(lr, a, false, inverse, s);
+    }
+  }
+  if (log_n >= 1 && log_n <= 5 && !pre && n_cols <= kTinyCols) {
+    const uint32_t nv = (uint32_t)n_valid;
+    switch (log_n) {
+      case 1: return tiny_ntt<1>(in, out, in_stride, out_stride, n_cols, nv, inverse, s);
+      case 2: return tiny_ntt<2>(in, out, in_stride, out_stride, n_cols, nv, inverse, s);
+      case 3: return tiny_ntt<3>(in, out, in_stride, out_stride, n_cols, nv, inverse, s);
+      case 4: return tiny_ntt<4>(in, out, in_stride, out_stride, n_cols, nv, inverse, s);
+      default: return tiny_ntt<5>(in, out, in_stride, out_stride, n_cols, nv, inverse, s);
     }
   }
   if (log_n <= 12) {

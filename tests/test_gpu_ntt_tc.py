@@ -48,6 +48,23 @@ def test_in_place(ctx, log_n, inverse):
         assert np.array_equal(got[c], O.ntt(x[c], inverse)), c
 
 
+# 2 .. 32 points, a thread a column: a warp's columns and one more, and both sides of the line
+# above which the shared-memory pass takes them; in place too
+@pytest.mark.parametrize("log_n", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("cols", [1, 6, 33, 32768, 32769])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_tiny(ctx, log_n, cols, inverse):
+    x = field(np.random.default_rng(log_n + cols), cols, 1 << log_n, "extreme" if cols == 33 else "random")
+    got = ctx.ntt(x, log_n, inverse)
+    for c in {0, cols // 2, cols - 1}:
+        assert np.array_equal(got[c], O.ntt(x[c], inverse)), c
+    d = torch.from_numpy(x.view(np.int64)).cuda()
+    torch.cuda.synchronize()
+    ctx.ntt(d, log_n, inverse, d)
+    torch.cuda.synchronize()
+    assert np.array_equal(d.cpu().numpy().view(np.uint64), got)
+
+
 # 2^11 .. 2^15 points: interleaved transforms and a radix stage (columns that share a
 # thread's powers in the stage's loop and a last ragged turn, one column, in place)
 @pytest.mark.parametrize("log_n,cols", [(11, 1), (11, 1200), (12, 1), (12, 301), (13, 2), (13, 160), (14, 1), (14, 75), (15, 3),
