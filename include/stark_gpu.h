@@ -92,6 +92,10 @@ const char* sg_last_error(const sg_ctx* ctx);
  * host round trip per fold layer). Each job's trace, LDE and constraint merge
  * still run on their own; every proof's bytes are unchanged. */
 #define SG_OPT_STIR_GROUP 2
+/* SG_OPT_FAULT: host-side fault injection for tests, SG_FAULT_* bits (default 0). Each raises
+ * the error on the host where the named step would have failed; no kernel is made to fail. */
+#define SG_OPT_FAULT 3
+#define SG_FAULT_STIR 1u /* the next STIR proof runs out of memory (SG_ENOMEM) with its first layer in the making */
 #define SG_WIDE_MERGE_AUTO 0
 #define SG_WIDE_MERGE_LDE 1
 #define SG_WIDE_MERGE_COSETS 2

@@ -262,6 +262,11 @@ int sg_ctx_set_option(sg_ctx* c, int option, int64_t value) {
     c->stir_group = (int)value;
     return SG_OK;
   }
+  if (option == SG_OPT_FAULT) {
+    if (value & ~(int64_t)SG_FAULT_STIR) return SG_EINVAL;
+    c->faults = (uint32_t)value;
+    return SG_OK;
+  }
   return SG_EINVAL;
 }
 

@@ -5,6 +5,7 @@
 // evaluations and the layer root (a few hundred bytes), derives the next
 // challenges, and finally gathers the s0 query openings in one copy.
 #include <algorithm>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -531,10 +532,13 @@ namespace {
 
 // A proof's stream s and the context's two side streams. Work on a side stream starts
 // after what `fork` saw on s; the destructor lets s wait for both, so that buffers (freed
-// in s's order) outlive what uses them, on every way out.
+// in s's order) outlive what uses them, on every way out. When it is an exception that
+// leaves, layers' results may still be on their way into the context's pinned staging, which
+// the next user fills from the host without a wait: then the host waits here.
 struct SideStreams {
   sg_ctx* c;
   cudaStream_t s, tree, ood;
+  const int exceptions = std::uncaught_exceptions();
   explicit SideStreams(sg_ctx* ctx) : c(ctx), s(ctx->stream) {
     int prio = 0;
     cuda_check(cudaStreamGetPriority(s, &prio), "stream priority");
@@ -560,6 +564,8 @@ struct SideStreams {
     cuda_check(cudaEventSynchronize(c->side_ev[4 + (ell & 1)]), "sync");
   }
   ~SideStreams() {
+    if (std::uncaught_exceptions() > exceptions)
+      for (cudaStream_t x : {tree, ood, s}) cudaStreamSynchronize(x);
     for (cudaStream_t x : {tree, ood})
       if (cudaEventRecord(c->side_ev[1], x) == cudaSuccess) cudaStreamWaitEvent(s, c->side_ev[1], 0);
   }
@@ -672,6 +678,10 @@ std::vector<uint8_t> stir_prove_on_stream(sg_ctx* c, const uint64_t* d_f0, uint6
     const unsigned lg = log2_exact(n);
     const bool last_cc = use_cc && ell == L - 1;
     start_ood(ell, zc);
+    if (c->faults & SG_FAULT_STIR) {
+      c->faults &= ~SG_FAULT_STIR;
+      throw SgError{SG_ENOMEM, "injected fault: STIR layer allocation failed"};
+    }
     if (ell > 0) take_layer(ell - 1);
     gl::Fp6 alpha = gl::e_zero();
     if (!last_cc) alpha = tr.challenge_ext("alpha");
