@@ -37,10 +37,11 @@ int guarded(sg_ctx* c, F&& f) {
   try {
     if (cudaSetDevice(c->device) != cudaSuccess) return fail(c, SG_ECUDA, "cudaSetDevice failed");
     f();
-    if (sg::ntt_tc_timed_out()) return fail(c, SG_ECUDA, "a bounded wait in a transform kernel ran out");
+    if (sg::wait_failed(c)) return fail(c, SG_ECUDA, sg::kWaitFailed);
     c->err.clear();
     return SG_OK;
   } catch (const sg::SgError& e) {
+    if (sg::wait_failed(c)) return fail(c, SG_ECUDA, sg::kWaitFailed);  // (a proof that does not verify, say)
     return fail(c, e.code, e.msg);
   } catch (const std::bad_alloc&) {
     return fail(c, SG_ENOMEM, "host allocation failed");
@@ -127,6 +128,15 @@ void pinned_release(sg_ctx* c) {
   c->pinned_bytes = 0;
 }
 
+bool wait_failed(sg_ctx* c) {
+  volatile int* f = c->tw.fail;
+  if (!f || !*f) return false;
+  for (cudaStream_t x : {c->stream, c->own_stream, c->stir_stream, c->side[0], c->side[1]})
+    if (x) cudaStreamSynchronize(x);
+  *f = 0;
+  return true;
+}
+
 void* pinned_host(sg_ctx* c, size_t bytes) {
   if (c->pinned_bytes >= bytes) return c->pinned;
   cuda_check(cudaStreamSynchronize(c->stream), "sync");  // no copy from the old buffer in flight
@@ -198,6 +208,7 @@ int sg_ctx_create(int device, sg_ctx** out) {
     delete c;
     return SG_ECUDA;
   }
+  c->tw.fail = sg::ntt_tc_fail_new();
   // Keep freed pool memory cached, so repeated proofs reuse it without cudaMalloc.
   // Never let the pool satisfy an allocation on one stream with a block freed on
   // another by making the first stream wait for the second: contexts proving
@@ -218,6 +229,7 @@ void sg_ctx_destroy(sg_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
+  int* const fail_word = c->tw.fail;
   if (c->owns_tables) sg::ntt_tables_free(&c->tw);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   if (c->copy_stream) {
@@ -238,6 +250,7 @@ void sg_ctx_destroy(sg_ctx* c) {
     if (x) cudaEventDestroy(x);
   if (c->stir_in) cudaEventDestroy(c->stir_in);
   if (c->stir_out) cudaEventDestroy(c->stir_out);
+  sg::ntt_tc_fail_free(fail_word);
   sg::pinned_release(c);
   delete c;
 }
@@ -263,8 +276,9 @@ int sg_ctx_set_option(sg_ctx* c, int option, int64_t value) {
     return SG_OK;
   }
   if (option == SG_OPT_FAULT) {
-    if (value & ~(int64_t)SG_FAULT_STIR) return SG_EINVAL;
+    if (value & ~(int64_t)(SG_FAULT_STIR | SG_FAULT_WAIT)) return SG_EINVAL;
     c->faults = (uint32_t)value;
+    if ((value & SG_FAULT_WAIT) && c->tw.fail) *(volatile int*)c->tw.fail = 1;
     return SG_OK;
   }
   return SG_EINVAL;

@@ -95,6 +95,11 @@ bool is_device_ptr(const void* p);
 // The context's pinned host staging buffer, grown to at least `bytes`. Earlier
 // contents are not kept; the caller synchronises its stream before the next use.
 void* pinned_host(sg_ctx* c, size_t bytes);
+// Whether a bounded wait ran out in a kernel of this context since the last call of this
+// function. If so its streams have been waited for and the word is clear again: the results
+// of the calls up to here are not to be used, later calls are not affected.
+bool wait_failed(sg_ctx* c);
+constexpr char kWaitFailed[] = "a bounded wait in a transform kernel ran out";
 // Give the context's staging buffer back to the process-wide pool.
 void pinned_release(sg_ctx* c);
 

@@ -34,6 +34,9 @@ struct NttTables {
   // byte matrices of the tensor-core passes (ntt_tc.cu), built per shape on first use;
   // null for callers that must not allocate
   TcCache* tc = nullptr;
+  // host-mapped word of this context's (tables may be shared), set by a tensor-core pass whose
+  // bounded wait ran out; without one these passes are not taken
+  int* fail = nullptr;
 };
 
 // Elements of one direction's block: st (4096) + lo + hi.

@@ -27,6 +27,7 @@
 #include <mutex>
 #include <new>
 #include <tuple>
+#include <vector>
 
 #include "counters.hpp"
 #include "gl.cuh"
@@ -97,18 +98,19 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
       : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
-// Waits for a phase with a limit. When it runs out, *abort is set for the CTA (later
-// waits return at once, so the CTA finishes its loops on data that nobody uses) and
-// the host is told through *fail.
-constexpr uint32_t kWaitLimit = 1u << 22;
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort, int* fail) {
-  for (uint32_t i = 0; i < kWaitLimit; ++i) {
-    if (mbar_try(bar, parity)) return;
-    if ((i & 63) == 63 && *abort) return;
-  }
-  *abort = 1;
+// Waits for a phase with a limit: 2^18 tries, each of which the hardware ends after 4 us, are
+// about a second. When it runs out, the host is told through *fail, and *pending = 1 + parity
+// says what is outstanding on the barrier: whoever issues for it issues nothing more and waits
+// for nothing, so that the loops run to their end on data that nobody uses, and the CTA waits
+// for it once more before it exits.
+constexpr uint32_t kWaitLimit = 1u << 18;
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* pending, int* fail) {
+  for (uint32_t i = 0; i < kWaitLimit; ++i)
+    if (mbar_try(bar, parity)) return true;
+  *pending = 1 + (int)parity;
   *(volatile int*)fail = 1;
   __threadfence_system();
+  return false;
 }
 
 __device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
@@ -278,7 +280,8 @@ __global__ void __launch_bounds__(Shape<LR1, LR2, PT>::T, LR1 == 4 && LR2 == 4 ?
   char* a_all = (char*)tw + S::TW_BYTES;
   char* tail = a_all + S::GROUPS * S::A_BYTES;
   uint32_t* tmem_slot = (uint32_t*)tail;
-  volatile int* abort = (volatile int*)(tail + 4);
+  // (mbar_wait) a group's products, then the tables
+  volatile int* pending = (volatile int*)(tail + 4);
   const uint32_t bars = smem_u32(tail + 16), tab_bar = bars + 8 * S::GROUPS;
   // the warp's number through a shuffle, so that what depends on it alone is uniform
   const int t = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, t >> 5, 0), grp = warp / (4 * PARTS);
@@ -295,8 +298,10 @@ __global__ void __launch_bounds__(Shape<LR1, LR2, PT>::T, LR1 == 4 && LR2 == 4 ?
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (t == 0) {
-    *abort = 0;
-    for (int g = 0; g <= S::GROUPS; ++g) mbar_init(bars + 8 * g, 1);
+    for (int g = 0; g <= S::GROUPS; ++g) {
+      pending[g] = 0;
+      mbar_init(bars + 8 * g, 1);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   tc_fence_before();
@@ -369,9 +374,11 @@ __global__ void __launch_bounds__(Shape<LR1, LR2, PT>::T, LR1 == 4 && LR2 == 4 ?
     }
   };
 
-  // one warp polls for the product, the others wait at the group's barrier
+  // the group's first warp issues its products and polls for them (until one fails to come), the
+  // others wait at the group's barrier
+  bool lead = gw == 0;
   auto wait_group = [&](uint32_t b, uint32_t parity) {
-    if (gw == 0) mbar_wait(b, parity, abort, a.fail);
+    if (lead) lead = __all_sync(0xFFFFFFFFu, mbar_wait(b, parity, pending + grp, a.fail));
     bar_group(1 + grp, S::GT);
     tc_fence_after();
   };
@@ -402,7 +409,7 @@ __global__ void __launch_bounds__(Shape<LR1, LR2, PT>::T, LR1 == 4 && LR2 == 4 ?
     }
     const char* q_tab = a.tab + S::B2_BYTES + (uint64_t)q * S::Q_BYTES;
     if (q != q_loaded) {
-      if (t == 0) {
+      if (t == 0 && pending[S::GROUPS] == 0) {
         const uint32_t bytes = PT == 2 ? S::B1_BYTES : S::Q_BYTES;
         mbar_expect(tab_bar, bytes + (q_loaded == ~0u ? S::B2_BYTES : 0));
         if (q_loaded == ~0u) bulk_load(b2_u, a.tab, S::B2_BYTES, tab_bar);
@@ -427,7 +434,8 @@ __global__ void __launch_bounds__(Shape<LR1, LR2, PT>::T, LR1 == 4 && LR2 == 4 ?
       __syncthreads();
     }
     if (q != q_loaded) {
-      mbar_wait(tab_bar, tab_phase, abort, a.fail);
+      if (pending[S::GROUPS] == 0) mbar_wait(tab_bar, tab_phase, pending + S::GROUPS, a.fail);
+      if (lead) lead = __all_sync(0xFFFFFFFFu, pending[S::GROUPS] == 0);
       tab_phase ^= 1;
       q_loaded = q;
     }
@@ -443,7 +451,7 @@ __global__ void __launch_bounds__(Shape<LR1, LR2, PT>::T, LR1 == 4 && LR2 == 4 ?
       fence_async_smem();
       tc_fence_before();
       bar_group(1 + grp, S::GT);
-      if (gw == 0) issue<R2 / 4, 8 * R1>(tmem, at_u, b1_u, bar);
+      if (lead) issue<R2 / 4, 8 * R1>(tmem, at_u, b1_u, bar);
       const uint32_t lane = min(g * L + l2, last_lane);
       char* o = at(out_q, y, a.out_colb);
       o = LF ? at(at(o, g, a.out_gb), lane - g * L, a.out_laneb) : at(o, lane, a.out_laneb);
@@ -473,7 +481,7 @@ __global__ void __launch_bounds__(Shape<LR1, LR2, PT>::T, LR1 == 4 && LR2 == 4 ?
       fence_async_smem();
       tc_fence_before();
       bar_group(1 + grp, S::GT);
-      if (gw == 0) issue<R1 / 4, 8 * R1>(tmem, at_u, b2_u, bar);
+      if (lead) issue<R1 / 4, 8 * R1>(tmem, at_u, b2_u, bar);
       uint64_t f = 0, rho = 0;
       if constexpr (PT == 1) {  // w_N^((j' + S i1) lane) g^lane as a geometric sequence in i1
         rho = tw_pow(a.tw_lo, a.tw_hi, (uint64_t)lane << a.log_s, a.pt_log);
@@ -505,6 +513,12 @@ __global__ void __launch_bounds__(Shape<LR1, LR2, PT>::T, LR1 == 4 && LR2 == 4 ?
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
+    // what was given up has its time once more to finish, before its memory is given back
+    if (t <= S::GROUPS && pending[t] != 0) {
+      for (uint32_t i = 0; i < kWaitLimit && !mbar_try(bars + 8 * t, pending[t] - 1); ++i) {
+      }
+    }
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*tmem_slot), "r"(S::GROUPS * S::COLS));
   }
 }
@@ -675,13 +689,13 @@ static cudaError_t build(const NttTables& t, const TcPass& a, bool inverse, char
 
 // False (and *a unchanged) when there is no room for the tables.
 bool ntt_tc_tables(const NttTables& t, TcPass* a, bool inverse, cudaStream_t s) {
-  if (!t.tc || !ntt_tc_ok(a->log_m) || !ntt_tc_fail_flag()) return false;
+  if (!t.tc || !t.fail || !ntt_tc_ok(a->log_m)) return false;
   const int lr1 = a->log_m == 10 ? 5 : 4, lr2 = a->log_m - lr1;
   const uint64_t bytes = image_bytes(lr1, lr2, a->n_q);
   if (bytes > kCacheBytes) return false;
   a->tw_lo = inverse ? t.d_inv_lo : t.d_fwd_lo;
   a->tw_hi = inverse ? t.d_inv_hi : t.d_fwd_hi;
-  a->fail = ntt_tc_fail_flag();
+  a->fail = t.fail;
   if (!a->pre.active()) {
     std::lock_guard<std::mutex> g(t.tc->mu);
     const auto key = std::make_tuple(a->log_m, a->log_s, a->n_q, a->j0, a->jq, a->jx, inverse, a->scale);
@@ -732,22 +746,42 @@ bool ntt_tc_tables(const NttTables& t, TcPass* a, bool inverse, cudaStream_t s) 
   return true;
 }
 
-int* ntt_tc_fail_flag() {
-  static int* flag = [] {
+// Words for contexts, 1024 (a page) allocated at a time and kept for the process: contexts
+// (a server's workers) come and go.
+namespace {
+struct FailWords {
+  std::mutex mu;
+  std::vector<int*> free;
+};
+FailWords& fail_words() {
+  static FailWords* w = new FailWords;
+  return *w;
+}
+}  // namespace
+
+int* ntt_tc_fail_new() {
+  FailWords& w = fail_words();
+  std::lock_guard<std::mutex> g(w.mu);
+  if (w.free.empty()) {
     int* p = nullptr;
-    if (cudaHostAlloc((void**)&p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+    constexpr int kWords = 1024;
+    if (cudaHostAlloc((void**)&p, kWords * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
       cudaGetLastError();
-      return (int*)nullptr;
+      return nullptr;
     }
-    *p = 0;
-    return p;
-  }();
-  return flag;
+    for (int i = kWords - 1; i >= 0; --i) w.free.push_back(p + i);
+  }
+  int* p = w.free.back();
+  w.free.pop_back();
+  *p = 0;
+  return p;
 }
 
-bool ntt_tc_timed_out() {
-  const int* f = ntt_tc_fail_flag();
-  return f && *(volatile const int*)f != 0;
+void ntt_tc_fail_free(int* p) {
+  if (!p) return;
+  FailWords& w = fail_words();
+  std::lock_guard<std::mutex> g(w.mu);
+  w.free.push_back(p);
 }
 
 void ntt_tc_drop(const TcPass& a, cudaStream_t s) {

@@ -50,10 +50,10 @@ bool ntt_tc_tables(const NttTables& t, TcPass* a, bool inverse, cudaStream_t s);
 void ntt_tc_drop(const TcPass& a, cudaStream_t s);
 // lanes_fast: a warp's accesses run over the lanes (in_lane or out_lane of 1) instead of along m and j'
 cudaError_t ntt_tc_pass(const TcPass& a, bool lanes_fast, cudaStream_t s);
-// host-mapped word that a kernel sets when a bounded wait ran out (null: no memory for it)
-int* ntt_tc_fail_flag();
-// true once a wait ran out in any kernel of this process: results since then are not to be used
-bool ntt_tc_timed_out();
+// A host-mapped word for NttTables::fail, zero (null: no memory for it), and its return once
+// no kernel runs that might set it.
+int* ntt_tc_fail_new();
+void ntt_tc_fail_free(int* p);
 
 TcCache* tc_cache_new();
 void tc_cache_free(TcCache* c);

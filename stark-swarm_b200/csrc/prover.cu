@@ -1147,8 +1147,8 @@ struct StirStreamScope {
 }  // namespace
 
 // A proof whose transforms ran out of a bounded wait is not handed out.
-static void check_waits() {
-  if (ntt_tc_timed_out()) throw SgError{SG_ECUDA, "a bounded wait in a transform kernel ran out"};
+static void check_waits(sg_ctx* c) {
+  if (wait_failed(c)) throw SgError{SG_ECUDA, kWaitFailed};
 }
 
 std::vector<uint8_t> stir_prove_device(sg_ctx* c, const uint64_t* d_f0, uint64_t n0, const sg_fri_params& p) {
@@ -1159,7 +1159,7 @@ std::vector<uint8_t> stir_prove_device(sg_ctx* c, const uint64_t* d_f0, uint64_t
     StirStreamScope scope(c);
     proof = stir_prove_on_stream(c, d_f0, n0, p);
   }
-  check_waits();
+  check_waits(c);
   return proof;
 }
 
@@ -1172,7 +1172,7 @@ std::vector<std::vector<uint8_t>> stir_prove_group(sg_ctx* c, const uint64_t* d_
     StirStreamScope scope(c);
     proofs = stir_prove_group_on_stream(c, d_f0, g_f0, n0, ps);
   }
-  check_waits();
+  check_waits(c);
   return proofs;
 }
 

@@ -25,6 +25,7 @@
 #include "p256.hpp"
 #include "p256_prover.hpp"
 #include "prover.hpp"
+#include "ntt_tc.cuh"
 #include "rsa2048.hpp"
 #include "sha256_air.cuh"
 #include "sha512_air.cuh"
@@ -320,6 +321,15 @@ struct sg_server {
       e->status = SG_EVERIFY;
       e->err = x.what();
     }
+    fail_on_wait(c, e);
+  }
+
+  // a job whose kernels gave up a wait did not fail for any other reason (and can be run again)
+  static void fail_on_wait(sg_ctx* c, Entry* e) {
+    if (!sg::wait_failed(c)) return;
+    e->status = SG_ECUDA;
+    e->err = sg::kWaitFailed;
+    e->proof.clear();
   }
 
   static void require_nonempty(const std::vector<uint8_t>& v) {
@@ -372,6 +382,7 @@ int sg_server_create(sg_ctx* ctx, int n_streams, uint64_t hbm_budget_bytes, sg_s
     sg_ctx* w = new sg_ctx;
     w->device = ctx->device;
     w->tw = ctx->tw;
+    w->tw.fail = sg::ntt_tc_fail_new();
     w->owns_tables = false;
     w->wide_merge = ctx->wide_merge;
     s->wctx.push_back(w);

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 import torch
 
+import oracle_lib as O
 import oracle_p256 as E
 
 pytestmark = pytest.mark.gpu
@@ -33,3 +34,31 @@ def test_staging_after_a_failed_stir_proof(sgpu):
         small = f0[:4096].contiguous()
         p = sgpu.build_params(4096, b"\2" * 32)
         assert sgpu.deep_fri_verify(p, c.deep_fri_prove(small, 4096, p))
+
+
+def test_a_wait_that_ran_out_is_the_context_s_own(sgpu):
+    """A kernel whose bounded wait ran out sets its context's word (here set from the host): that
+    context's next call reports it, no other context's does, nor that context's later ones."""
+    x = np.random.default_rng(1).integers(0, O.P, size=(3, 1 << 10), dtype=np.uint64)
+    want = np.stack([O.ntt(c) for c in x])
+    msg, pi = b"one record", b"\1" * 32
+    p = sgpu.build_params(4096, pi)
+    f0 = np.arange(4096, dtype=np.uint64)
+    with sgpu.Context(0) as c, sgpu.Context(0) as other:
+        proof, digest = other.prove_sha256(msg, pi)
+        stir = other.deep_fri_prove(f0, 4096, p)
+        calls = [
+            (lambda: c.ntt(x, 10, False).tolist(), want.tolist()),
+            (lambda: c.prove_sha256(msg, pi), (proof, digest)),
+            (lambda: c.deep_fri_prove(f0, 4096, p), stir),
+            (lambda: c.deep_fri_prove_group(np.stack([f0, f0]), [p, p]), [stir, stir]),
+        ]
+        for call, result in calls:
+            c.set_option(sgpu.OPT_FAULT, sgpu.FAULT_WAIT)
+            assert np.array_equal(other.ntt(x, 10, False), want)
+            # a server's workers are contexts of their own
+            assert c.prove_batch([(sgpu.JOB_SHA256, msg, pi)], n_streams=2)[0][0] == proof
+            with pytest.raises(sgpu.StarkGpuError) as ei:
+                call()
+            assert ei.value.code == sgpu.SG_ECUDA and "wait" in str(ei.value)
+            assert call() == result
