@@ -342,7 +342,8 @@ def build_params(n0: int, pk_hash_32: bytes = None, stir: bool = True) -> FriPar
 
 
 def ntt_set_split(log_n: int, padded: bool, log_n1: int):
-    """sg_ntt_set_split: pin the four-step split of 2^log_n transforms (0 = default)."""
+    """sg_ntt_set_split: pin the four-step split of 2^log_n transforms (0 or log_n // 2 = default);
+    restores what Context.ntt_autotune returned."""
     rc = lib().sg_ntt_set_split(log_n, int(padded), log_n1)
     if rc != SG_OK:
         raise StarkGpuError(rc, "sg_ntt_set_split: size or split out of range")

@@ -318,6 +318,7 @@ int sg_ntt_autotune(sg_ctx* c, size_t n_cols, size_t log_n, int inverse, size_t 
     try {
       for (int k = lo; k <= hi + 1; ++k) {
         const int l1 = k <= hi ? k : 0;
+        if (l1 == (int)log_n / 2) continue;  // names no pin
         sg::ntt_set_split((int)log_n, padded, l1);
         auto run = [&] {
           sg::cuda_check(sg::ntt_batch(c->tw, in.p, out.p, (uint32_t)cols, N, N, (int)log_n, inverse != 0, n_valid,

@@ -964,6 +964,7 @@ static int ntt_split(int log_n, bool padded, int le, bool tc) {
 }
 
 void ntt_set_split(int log_n, bool padded, int log_n1) {
+  if (log_n1 == log_n / 2) log_n1 = 0;  // what ntt_split says of no pin
   if (log_n >= 13 && log_n <= 24) g_split[log_n][padded ? 1 : 0].store(log_n1);
 }
 
