@@ -236,8 +236,9 @@ int sg_prove_sha512(sg_ctx* ctx, const uint8_t* msg, size_t len, const uint8_t f
  * padding, for every later transform in the process (all splits give the same
  * output). The default without a pinned split, whose passes a split may not have, is timed
  * too and stays when it is within 2 % of the fastest. best_log_n1 (optional) receives log N1
- * of the chosen split, log N / 2 (rounded down) for the default. Call it
- * before the timed or latency-sensitive work, like cuDNN's benchmark mode. */
+ * of the chosen split, log N / 2 (rounded down) for the default. A pinned split concerns
+ * single transforms; sg_lde onto up to 2^24 points from 2^11 .. 2^20 rows has passes of its
+ * own. Call it before the timed or latency-sensitive work, like cuDNN's benchmark mode. */
 int sg_ntt_autotune(sg_ctx* ctx, size_t n_cols, size_t log_n, int inverse, size_t n_valid, int* best_log_n1);
 /* Set the split directly (a saved sg_ntt_autotune result; 0 and log N / 2 = the default, none pinned):
  * SG_EINVAL unless 13 <= log_n <= 24 and max(1, log_n - 12) <= log_n1 <= min(12, log_n - 1). */

@@ -1243,8 +1243,8 @@ cudaError_t ntt_lde(const NttTables& t, const uint64_t* in, uint64_t* coef, uint
   if (t.tc && radix_size(log_n) && log_b >= 1 && n_cols > 0)
     return lde_radix(t, in, coef, out, n_cols, log_n, log_b, s, pre);
   const int log_e = log_n + log_b, l1 = log_n / 2, l2 = log_n - l1;
-  if (!t.tc || !ntt_tc_ok(l1) || !ntt_tc_ok(l2) || log_b < 1 || log_e > 24 || !scratch || n_cols == 0 ||
-      g_split[log_n][0].load() || g_split[log_e][1].load())
+  // (a pinned split is one of ntt_batch's four-step transforms, which these are not)
+  if (!t.tc || !ntt_tc_ok(l1) || !ntt_tc_ok(l2) || log_b < 1 || log_e > 24 || !scratch || n_cols == 0)
     return cudaErrorNotSupported;
   const uint64_t n = 1ull << log_n;
   TcPass p[4] = {ntt_tc_args(l2, 0), ntt_tc_args(l1, 0), ntt_tc_args(l1, log_b), ntt_tc_args(l2, 0)};

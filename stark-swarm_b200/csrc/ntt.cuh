@@ -93,7 +93,7 @@ cudaError_t ntt_batch(const NttTables& t, const uint64_t* in, uint64_t* out, uin
 // points, as ntt_batch's inverse and then its zero-padded forward transform with `pre`, for
 // traces of 2^11 .. 2^20 rows; coef (n_cols 2^log_n elements) holds the coefficients in an
 // order of its own. cudaErrorNotSupported (nothing done) when these transforms do not run
-// on the tensor cores or, from 2^16 rows, a split is pinned.
+// on the tensor cores.
 // scratch (from 2^16 rows): ntt_scratch_elems(n_cols, log_n + log_b).
 cudaError_t ntt_lde(const NttTables& t, const uint64_t* in, uint64_t* coef, uint64_t* out, uint32_t n_cols, int log_n,
                     int log_b, uint64_t* scratch, cudaStream_t s, const PowSpec* pre = nullptr);
