@@ -95,8 +95,9 @@ const char* sg_last_error(const sg_ctx* ctx);
 /* SG_OPT_FAULT: host-side fault injection for tests, SG_FAULT_* bits (default 0). Each raises
  * the error on the host where the named step would have failed; no kernel is made to fail. */
 #define SG_OPT_FAULT 3
-#define SG_FAULT_WAIT 2u /* the next call finds that a bounded wait in a transform kernel ran out (SG_ECUDA) */
 #define SG_FAULT_STIR 1u /* the next STIR proof runs out of memory (SG_ENOMEM) with its first layer in the making */
+#define SG_FAULT_WAIT 2u /* the next call finds that a bounded wait in a transform kernel ran out (SG_ECUDA) */
+#define SG_FAULT_TABLES 4u /* while set, transforms find no memory for their tables (and run without them) */
 #define SG_WIDE_MERGE_AUTO 0
 #define SG_WIDE_MERGE_LDE 1
 #define SG_WIDE_MERGE_COSETS 2

@@ -151,7 +151,7 @@ OPT_WIDE_MERGE = 1
 OPT_STIR_GROUP = 2  # servers from this context prove up to this many same-n0 STIR phases in lockstep
 WIDE_MERGE_AUTO, WIDE_MERGE_LDE, WIDE_MERGE_COSETS = 0, 1, 2
 OPT_FAULT = 3  # host-side fault injection for tests
-FAULT_STIR, FAULT_WAIT = 1, 2
+FAULT_STIR, FAULT_WAIT, FAULT_TABLES = 1, 2, 4
 
 
 class Job(ctypes.Structure):

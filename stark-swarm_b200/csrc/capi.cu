@@ -276,8 +276,9 @@ int sg_ctx_set_option(sg_ctx* c, int option, int64_t value) {
     return SG_OK;
   }
   if (option == SG_OPT_FAULT) {
-    if (value & ~(int64_t)(SG_FAULT_STIR | SG_FAULT_WAIT)) return SG_EINVAL;
+    if (value & ~(int64_t)(SG_FAULT_STIR | SG_FAULT_WAIT | SG_FAULT_TABLES)) return SG_EINVAL;
     c->faults = (uint32_t)value;
+    c->tw.no_room = (value & SG_FAULT_TABLES) != 0;
     if ((value & SG_FAULT_WAIT) && c->tw.fail) *(volatile int*)c->tw.fail = 1;
     return SG_OK;
   }

@@ -880,8 +880,7 @@ cudaError_t ntt_coset_eval(const NttTables& t, const uint64_t* coef, uint64_t* o
     p.pre = pre ? *pre : PowSpec{};
     if (ntt_tc_tables(t, &p, false, s)) return ntt_tc_pass(p, false, s);
   }
-  // fewer cosets than a lane-per-coset pass's lanes
-  if (log_b < pass_log_k(log_m)) return t.tc ? cudaErrorMemoryAllocation : cudaErrorInvalidValue;
+  if (log_b < pass_log_k(log_m)) return cudaErrorNotSupported;  // fewer cosets than a lane-per-coset pass's lanes
   PassArgs a = base_args(t, false);
   a.pre = pre ? *pre : PowSpec{};
   a.in = coef;

@@ -37,6 +37,7 @@ struct NttTables {
   // host-mapped word of this context's (tables may be shared), set by a tensor-core pass whose
   // bounded wait ran out; without one these passes are not taken
   int* fail = nullptr;
+  bool no_room = false;  // (tests) as if there were no memory for the byte matrices
 };
 
 // Elements of one direction's block: st (4096) + lo + hi.
@@ -103,7 +104,8 @@ cudaError_t ntt_lde(const NttTables& t, const uint64_t* in, uint64_t* coef, uint
 // (column stride N) in one pass, without scratch: a forward transform of the
 // zero-padded coefficients times g^k, as ntt_batch computes it with `pre`.
 // Needs ntt_coset_eval_ok(log_m, log_b): log_m <= 10 and N >= 2^8, or log_m <= 12 and at
-// least as many cosets as a pass's lanes per CTA.
+// least as many cosets as a pass's lanes per CTA. cudaErrorNotSupported (nothing done) with
+// fewer cosets than those when there is no room for the tensor-core tables.
 bool ntt_coset_eval_ok(int log_m, int log_b);
 cudaError_t ntt_coset_eval(const NttTables& t, const uint64_t* coef, uint64_t* out, uint32_t n_cols, int log_m,
                            int log_b, cudaStream_t s, const PowSpec* pre = nullptr);

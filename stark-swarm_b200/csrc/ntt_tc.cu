@@ -689,7 +689,7 @@ static cudaError_t build(const NttTables& t, const TcPass& a, bool inverse, char
 
 // False (and *a unchanged) when there is no room for the tables.
 bool ntt_tc_tables(const NttTables& t, TcPass* a, bool inverse, cudaStream_t s) {
-  if (!t.tc || !t.fail || !ntt_tc_ok(a->log_m)) return false;
+  if (!t.tc || !t.fail || t.no_room || !ntt_tc_ok(a->log_m)) return false;
   const int lr1 = a->log_m == 10 ? 5 : 4, lr2 = a->log_m - lr1;
   const uint64_t bytes = image_bytes(lr1, lr2, a->n_q);
   if (bytes > kCacheBytes) return false;

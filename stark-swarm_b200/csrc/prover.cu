@@ -105,11 +105,17 @@ void lde_core(sg_ctx* c, const uint64_t* d_trace, uint64_t w, uint64_t n_trace, 
     return;
   }
   ntt(c, d_trace, coef, (uint32_t)w, n_trace, n_trace, log2_exact(n_trace), true, n_trace, scratch);
+  DBuf own;
   if (lde_by_cosets(n_trace, blowup)) {
-    cuda_check(ntt_coset_eval(c->tw, coef, d_out, (uint32_t)w, (int)log2_exact(n_trace), (int)log2_exact(blowup),
-                              c->stream, sh.active ? &sh.spec : nullptr),
-               "coset evaluation");
-    return;
+    const cudaError_t ec = ntt_coset_eval(c->tw, coef, d_out, (uint32_t)w, (int)log2_exact(n_trace),
+                                          (int)log2_exact(blowup), c->stream, sh.active ? &sh.spec : nullptr);
+    if (ec != cudaErrorNotSupported) {
+      cuda_check(ec, "coset evaluation");
+      return;
+    }
+    // no room for its tables: the padded transform, whose scratch the caller has not reserved
+    own.alloc(ntt_scratch_elems(w, log2_exact(n0)), c->stream);
+    scratch = own.p;
   }
   ntt(c, coef, d_out, (uint32_t)w, n_trace, n0, log2_exact(n0), false, n_trace, scratch,
       sh.active ? &sh.spec : nullptr);

@@ -62,3 +62,39 @@ def test_a_wait_that_ran_out_is_the_context_s_own(sgpu):
                 call()
             assert ei.value.code == sgpu.SG_ECUDA and "wait" in str(ei.value)
             assert call() == result
+
+
+# LDEs that run as one tensor-core pass (rows of 2^8 .. 2^10, or fewer onto 2^11 points), with
+# fewer and with more cosets than a lane-per-coset pass has lanes; in interleaved parts (2^11
+# .. 2^15 rows); in blocks (2^16 rows)
+@pytest.mark.parametrize("log_n,blowup", [(3, 256), (5, 64), (7, 16), (7, 32), (8, 2), (8, 4), (8, 64), (9, 2),
+                                          (9, 8), (9, 32), (10, 2), (10, 4), (10, 8), (10, 32), (11, 2), (11, 32), (13, 4),
+                                          (15, 2), (16, 8)])
+@pytest.mark.parametrize("shift", [1, 7])
+def test_lde_without_room_for_tables(sgpu, log_n, blowup, shift):
+    x = np.random.default_rng(log_n).integers(0, O.P, size=(3, 1 << log_n), dtype=np.uint64)
+    with sgpu.Context(0) as c:
+        c.set_option(sgpu.OPT_FAULT, sgpu.FAULT_TABLES)
+        assert np.array_equal(c.lde(x, blowup, shift), O.lde(x, blowup, shift))
+
+
+@pytest.mark.parametrize("log_n", [8, 9, 10, 11, 12, 13, 15, 16, 17, 20, 21, 22])
+def test_ntt_without_room_for_tables(sgpu, log_n):
+    x = np.random.default_rng(log_n).integers(0, O.P, size=(2, 1 << log_n), dtype=np.uint64)
+    with sgpu.Context(0) as c:
+        c.set_option(sgpu.OPT_FAULT, sgpu.FAULT_TABLES)
+        for inverse in (False, True):
+            assert np.array_equal(c.ntt(x, log_n, inverse), np.stack([O.ntt(col, inverse) for col in x]))
+
+
+def test_proofs_without_room_for_tables(sgpu):
+    rng = random.Random(2)
+    a, b = [rng.randrange(2) for _ in range(256)], [rng.randrange(2) for _ in range(256)]
+    _, q = E.keypair(0x1357)
+    pi = b"\3" * 32
+    with sgpu.Context(0) as c, sgpu.Context(0) as free:
+        c.set_option(sgpu.OPT_FAULT, sgpu.FAULT_TABLES)
+        c.set_option(sgpu.OPT_WIDE_MERGE, sgpu.WIDE_MERGE_COSETS)
+        assert c.prove_sha256(b"x" * 64, pi) == free.prove_sha256(b"x" * 64, pi)
+        assert c.prove_sha512(b"x" * 300, pi) == free.prove_sha512(b"x" * 300, pi)
+        assert c.prove_p256_chains(E.G, a, q, b, pi) == free.prove_p256_chains(E.G, a, q, b, pi)
