@@ -730,11 +730,12 @@ RadixArgs radix_args(const NttTables& t, const uint64_t* in, uint64_t in_col, ui
 }
 
 // A transform of 2 .. 32 points by one thread: a thread a column, no twiddle and no exchange.
-// A launch of few columns is bound by its latency: a call of 6 x 2^4 takes 13 us where the
-// shared-memory pass took 19, 11041 x 2^5 (an RSA trace) 19.6 and 21.4. Each thread walks its
-// own lines, so the gain goes with the columns (40000 x 2^4: 19.2 and 20.1); above kTinyCols
-// the pass that loads whole tiles stays.
-constexpr uint32_t kTinyCols = 32768;
+// A launch of few columns is bound by its latency: an inverse of 6 x 2^4 takes 13.6 us as a
+// call where the shared-memory pass takes 19.4, 12288 x 2^5 (an RSA trace has 11041) 19.7 and
+// 21.6. Each thread walks its own lines, so the gain goes with the columns: 16384 x 2^5 20.8 and
+// 21.7 us, but 24576 x 2^5 22.5 and 21.5; 32768 x 2^4 17.8 and 20.3, 49152 x 2^4 20.2 and 20.2;
+// 32768 x 2^3 14.9 and 19.9. Above these lines the pass that loads whole tiles stays.
+constexpr uint32_t tiny_cols(int log_n) { return log_n == 5 ? 16384 : 32768; }
 template <int LR, bool INV>
 __global__ void __launch_bounds__(32) tiny_ntt_kernel(const uint64_t* in, uint64_t* out, uint64_t in_stride,
                                                       uint64_t out_stride, uint32_t n_cols, uint32_t n_valid) {
@@ -1029,7 +1030,7 @@ cudaError_t ntt_batch(const NttTables& t, const uint64_t* in, uint64_t* out, uin
       return radix_pass(lr, a, false, inverse, s);
     }
   }
-  if (log_n >= 1 && log_n <= 5 && !pre && n_cols <= kTinyCols) {
+  if (log_n >= 1 && log_n <= 5 && !pre && n_cols <= tiny_cols(log_n)) {
     const uint32_t nv = (uint32_t)n_valid;
     switch (log_n) {
       case 1: return tiny_ntt<1>(in, out, in_stride, out_stride, n_cols, nv, inverse, s);

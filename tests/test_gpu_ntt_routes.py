@@ -79,3 +79,14 @@ def test_pinned_padded_splits(sgpu, ctx, log_n):
             assert np.array_equal(run(), want), l1
         finally:
             sgpu.ntt_set_split(log_n, True, 0)
+
+
+@pytest.mark.parametrize("log_n,most", [(1, 32768), (4, 32768), (5, 16384)])
+def test_tiny_transforms_up_to_their_line(sgpu, ctx, log_n, most):
+    """A thread a column as far as it is the faster one; the results on both sides of the line."""
+    for cols, name in ((most, "ntt_radix"), (most + 1, "ntt_pass")):
+        x = field(cols, 1 << log_n, cols)
+        got = []
+        assert launches(sgpu, lambda: got.append(ctx.ntt(x, log_n, True))) == {name: 1}
+        for c in (0, cols // 2, cols - 1):
+            assert np.array_equal(got[0][c], O.ntt(x[c], True)), c
