@@ -152,14 +152,13 @@ class ClockSampler:
 #   inverse 2^20, pass 1: 168.9 us, 225 MB; pass 2: 87.8 us, 221 MB
 #   forward 2^23, pass 1: 827 us, 2.11 GB: ALU 42 %, FMA 52 %, tensor 31 %
 #   forward 2^23, pass 2: 753 us, 2.10 GB: ALU 33 %, FMA 40 %, tensor 34 %
-# leaf_kernel_t<64> (2^20 rows of 64 columns): ALU 83.2 % at 1.489 ms, before its rounds
-# were rolled (1.405 ms)
+# leaf_kernel_t<64> (2^20 rows of 64 columns): 1.415 ms, ALU 85.7 %, FMA 42.7 %, 0.57 GB
 _LDE_TRAFFIC = (225e6 + 221e6 + 2.11e9 + 2.10e9) * 4  # bytes per 64-column LDE (4 launches)
 MEASURED_NTT = {
     "ntt_pass": {"int_frac": 0.38, "int_metric": "ALU-pipe share of active cycles (ncu, 16-column case); FMA pipe 0.46, "
                                                  "tensor pipe 0.33",
                  "traffic_per_lde": _LDE_TRAFFIC},
-    "merkle_leaves": {"int_frac": 0.832, "int_metric": "ALU-pipe share of active cycles (ncu, 2^20 x 64 leaves)"},
+    "merkle_leaves": {"int_frac": 0.857, "int_metric": "ALU-pipe share of active cycles (ncu, 2^20 x 64 leaves)"},
 }
 # DRAM bytes per step of the ntt_pass family: the LDE's (above) plus the STIR
 # proof's transforms, taken at their algorithmic bytes times the LDE's

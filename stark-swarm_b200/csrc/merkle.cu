@@ -228,10 +228,9 @@ __device__ void node_hash_warp(const uint64_t* child, uint64_t n_child, uint64_t
 // spreads over all SMs. The last levels, of at most kTopNodes parents: one CTA, a warp per
 // node and a barrier (which makes the level's global writes visible to the whole block)
 // between the levels, which saves their launches. A node's one to five permutations are one
-// after another, about 2.5 us each with its loads, and that chain is the whole time. Up to
-// now all levels of at most 1024 permutations ran in one CTA, most by a thread a node: the
-// trees of a 64-byte SHA-256 proof took 325 us of kernel time and take 267, those of a
-// 512-point rollup 148 and 121.
+// after another, about 2.5 us each with its loads, and that chain is the whole time. Against
+// all levels of at most 1024 permutations in one CTA, most by a thread a node: the trees of a
+// 64-byte SHA-256 proof 267 us of kernel time (325), those of a 512-point rollup 121 (148).
 constexpr uint64_t kWarpNodes = 1024, kTopNodes = 16;
 constexpr int kTopThreads = 32 * (int)kTopNodes, kWarpNodeThreads = 64;
 constexpr int kMaxTopLevels = 24;

@@ -14,12 +14,14 @@
 // E > 1 evaluating E M points from M coefficients (zero padding, coset LDE): the
 // first matrix of a chunk of R1 values of j' carries the coset shift and 1/N too.
 //
-// What bounds it: the integer pipes of the epilogues (per output two digit joins of 13
-// instructions and one product of 15), at 40-65 % of their issue rate; the tensor pipe is
-// active 25 % (R1 = 16) to 45 % (R1 = 32) of the time, HBM 20-30 %. Measured (one call, device
-// tensors, before = the radix-16 butterfly passes of ntt.cu, after): LDE of 4099 x 1024
-// points x 32: 1666 -> 600 us; 20000 x 256 x 32: 1588 -> 595 us; 64 x 2^20 x 8:
-// 14.7 -> 7.0 ms; inverse 6 x 2^20: 178 -> 130 us; one column of 2^8: 25 -> 19 us.
+// What bounds it: a tile's serial chain (load, product, join, twiddle, product, join, store),
+// of which an SM holds two tiles (R1 = 32) or four (R1 = 16); their accumulators fill its
+// tensor memory. No pipe is full: 32 x 32 has the FMA pipe active 37-52 %, ALU 30-42 %, tensor
+// 22-39 % of the time; 16 x 16, in bulk, FMA 62 %, ALU 51 %, tensor 26 %. Measured (one call,
+// device tensors, before = the radix-16 butterfly passes of ntt.cu, after): LDE of 4099 x 1024
+// points x 32: 1666 -> 662 us (600 on buffers that the call before used); 756 x 256 x 32:
+// 102 -> 53 us; 64 x 2^20 x 8: 14.7 -> 7.1 ms; inverse 6 x 2^20: 177 -> 123 us; one column of
+// 2^8: 25 -> 19 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -795,8 +797,10 @@ cudaError_t ntt_tc_pass(const TcPass& a, bool lanes_fast, cudaStream_t s) {
     return cudaSuccess;
   }
   // The lane tables of PT = 2 cost about as much as a pair of tiles, so they are shared by at
-  // least 8 columns, and there have to be two waves of such units (6 x 2^20: 138 us with
-  // them, 128 without; 100 x 2^14: 67 and 51; 64 x 2^20: 934 and 979).
+  // least 8 columns, and there have to be two waves of such units. Inverse transforms with
+  // them and without: 8 x 2^20 157 and 149 us, 32 x 2^20 491 and 500, 64 x 2^20 910 and 962; 16
+  // x 2^18 79 and 76, 64 x 2^18 235 and 238, 320 x 2^18 969 and 1037; 80 x 2^16 78 and 78, 320
+  // x 2^16 222 and 222. (From two to some four waves they cost up to 6 %, 16 x 2^20 282 and 266.)
   const uint64_t units = (uint64_t)(a.n_lanes / ntt_tc_lanes(a.log_m)) * a.n_q * (a.n_y / 8);
   const int pt = a.pt_log == 0 ? 0 : units < 2 * 148 * (a.log_m == 8 ? 2 : 1) ? 1 : 2;
   cudaError_t e = cudaErrorInvalidValue;
